@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
     // ended finishes it and starts the next in the same iteration.
     bool live = start();
     while (__any_sync(0xffffffffu, live)) {
-        if (!live) continue;
-        bool go = step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
+        bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
+        __syncwarp();          // join locate()'s exits before the update (track_step)
         if (go) {
             update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng);
             s.steps += 1u;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
                 step += 1u;
             }
         }
-        if (!go) {
+        if (live && !go) {
             finish();
             live = start();
         }

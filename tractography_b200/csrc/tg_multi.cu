@@ -83,8 +83,8 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
 #pragma unroll
     for (int k = 0; k < CPAD; ++k) c[k] = 0.0f;
     unsigned long long steps_total = 0;
-    const JobDev* J = nullptr;
-    const TrackParams* P = nullptr;
+    const JobDev* J = mp.jobs;
+    const TrackParams* P = &J->t;
     Lane s;
     int32_t chunk = -1;
     uint32_t fill = 0;
@@ -143,21 +143,18 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
                 lane_save<ALGO != kTransport>(mp.carry_out + atomicAdd(mp.carry_out_count, 1u), s, g, chunk, fill);
             break;
         }
+        float qx, qy, qz;
+        const bool go = live && s.n < P->n_steps && s.steps < P->max_steps;
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD>(*P, go, s, c, qx, qy, qz);
         if (!live) continue;
-        bool done = s.n >= P->n_steps || s.steps >= P->max_steps;
+        bool done = r == 0;
         bool overflow = false;
-        if (!done) {
-            float qx, qy, qz;
-            const int r = track_step<MODEL, LMAX, ALGO, CPAD>(*P, s, c, qx, qy, qz);
-            if (r == 0) {
+        if (r == 2) {
+            if (m_emit(mp, chunk, fill, qx, qy, qz)) {
+                s.n++;
+            } else {
                 done = true;
-            } else if (r == 2) {
-                if (m_emit(mp, chunk, fill, qx, qy, qz)) {
-                    s.n++;
-                } else {
-                    done = true;
-                    overflow = true;
-                }
+                overflow = true;
             }
         }
         if (done) {

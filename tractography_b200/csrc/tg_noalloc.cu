@@ -71,28 +71,36 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
     float c[CPAD];
 #pragma unroll
     for (int k = 0; k < CPAD; ++k) c[k] = 0.0f;
-    while (true) {
+    Lane s;
+    uint32_t item = 0;
+    float4* line = out;
+    auto fetch = [&]() -> bool {
         const unsigned long long it = atomicAdd(item_counter, 1ull);
-        if (it >= n_seeds) break;
-        const uint32_t item = (uint32_t)it;
+        if (it >= n_seeds) return false;
+        item = (uint32_t)it;
         const uint32_t batch = item / batch_size;
         const uint32_t local = item - batch * batch_size;
         const float4 a = seeds[2 * (size_t)item];
         const float4 b = seeds[2 * (size_t)item + 1];
-        Lane s;
         lane_init(s, a, b, batch_seeds[batch], local, seed_offset + item);
-        float4* line = out + (size_t)item * p.n_steps;
+        line = out + (size_t)item * p.n_steps;
         line[0] = a;
-        while (s.n < p.n_steps && s.steps < p.max_steps) {
-            float qx, qy, qz;
-            const int r = track_step<MODEL, LMAX, ALGO, CPAD>(p, s, c, qx, qy, qz);
-            if (r == 0) break;
-            if (r == 2) {
-                line[s.n] = make_float4(qx, qy, qz, 1.0f);
-                s.n++;
-            }
+        return true;
+    };
+    bool live = fetch();
+    while (__any_sync(0xffffffffu, live)) {
+        float qx, qy, qz;
+        const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD>(p, go, s, c, qx, qy, qz);
+        if (!live) continue;
+        if (r == 2) {
+            line[s.n] = make_float4(qx, qy, qz, 1.0f);
+            s.n++;
         }
-        lengths[item] = s.n;
+        if (r == 0) {
+            lengths[item] = s.n;
+            live = fetch();
+        }
     }
 }
 

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
     const uint32_t avail = sp.P.alloc[0];
     Lane s;
     s.px = s.py = s.pz = 0.0f;
-    const ServeJob* J = nullptr;
+    const ServeJob* J = sp.jobs;
     uint32_t slot = 0, item = 0, fill = 0;
     int32_t chunk = -1;
     uint32_t budget = sp.step_budget;
@@ -261,21 +261,18 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             break;
         }
         budget -= 1u;
+        float qx, qy, qz;
+        const bool go = live && s.n < J->t.n_steps && s.steps < J->t.max_steps;
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(J->t, go, s, c, qx, qy, qz);
         if (!live) continue;
-        bool done = s.n >= J->t.n_steps || s.steps >= J->t.max_steps;
+        bool done = r == 0;
         bool overflow = false;
-        if (!done) {
-            float qx, qy, qz;
-            const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(J->t, s, c, qx, qy, qz);
-            if (r == 0) {
+        if (r == 2) {
+            if (s_emit(sp.P, avail, chunk, fill, qx, qy, qz)) {
+                s.n++;
+            } else {
                 done = true;
-            } else if (r == 2) {
-                if (s_emit(sp.P, avail, chunk, fill, qx, qy, qz)) {
-                    s.n++;
-                } else {
-                    done = true;
-                    overflow = true;
-                }
+                overflow = true;
             }
         }
         if (done) {

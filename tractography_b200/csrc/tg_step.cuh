@@ -49,14 +49,11 @@ struct Lane {
     uint32_t seed_state;
 };
 
-// One iteration of tracking.py:121-147 after the n < N_STEPS test.
-// Returns 0 when the streamline stops (domain or field check failed),
-// 1 after a step without a saved point, 2 after a step that saved point q.
-//
 // DOM selects the domain test: the image mask (domain.py:358-382), or a
 // closed surface, where the seed must be inside and every later point must
 // be reached by a segment from the previous one that does not hit the
 // surface (the found flag of bvh.cl:83-131).
+//
 // The domain test and the field gather of one iteration (tracking.py:123-
 // 133): false when the streamline stops; otherwise c holds the coefficients
 // of the nearest field voxel.
@@ -197,11 +194,25 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
     return true;
 }
 
+// One iteration of tracking.py:121-147 after the n < N_STEPS test.
+// Returns 0 when the streamline stops (domain or field check failed, or go
+// is false), 1 after a step without a saved point, 2 after a step that saved
+// point q.
+//
+// Called by all 32 lanes of a warp together; lanes without a step to make
+// pass go = false.  locate() has many exits (voxel unchanged, voxel loaded,
+// stopped), and left to itself the compiler joins its paths only behind the
+// update, which then ran once per path: with a 0.1-voxel step some lane of
+// nearly every warp enters a new voxel on every step, and 11-13 of 32 lanes
+// were active per instruction (~1000 warp instructions per step).  The
+// __syncwarp joins the lanes before the update.
 template <int MODEL, int LMAX, int ALGO, int CPAD, int DOM = kDomainImage>
-__device__ __forceinline__ int track_step(const TrackParams& p, Lane& s, float (&c)[CPAD],
+__device__ __forceinline__ int track_step(const TrackParams& p, bool go, Lane& s, float (&c)[CPAD],
                                           float& qx, float& qy, float& qz, int surface = -1)
 {
-    if (!locate<MODEL, LMAX, CPAD, DOM>(p, s, c, surface)) return 0;
+    if (go) go = locate<MODEL, LMAX, CPAD, DOM>(p, s, c, surface);
+    __syncwarp();
+    if (!go) return 0;
     update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng);
     s.steps += 1u;
 

@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
     // lanes until the warp's longest track ends).
     bool live = start();
     while (__any_sync(0xffffffffu, live)) {
-        if (!live) continue;
-        bool go = step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
+        bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
+        __syncwarp();          // join locate()'s exits before the update (track_step)
         if (go) {
             // output voxel nearest the point, floor(A^-1 p + 0.5) (tracking.py:294-300)
             const float vx = floorf(dot4(q.out_row0, s.px, s.py, s.pz, 1.0f) + 0.5f);
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
                 step += 1u;
             }
         }
-        if (!go) {
+        if (live && !go) {
             if (prev_x >= 0) tod_flush(q.coefficients, acc, tid, prev_x, prev_y, prev_z, q);
             steps_total += s.steps;
             live = start();

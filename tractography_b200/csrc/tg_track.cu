@@ -41,26 +41,30 @@ __global__ void __launch_bounds__(128) track_dense_kernel(TrackParams p, const f
 {
     constexpr int CPAD = ModelShape<MODEL, LMAX>::CPAD;
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= n_seeds) return;
+    const bool own = gid < n_seeds;
     Lane s;
-    const float4 a = seeds[2 * (size_t)gid];
-    const float4 b = seeds[2 * (size_t)gid + 1];
+    const size_t row = own ? gid : 0;      // lanes past the end keep their warp whole and track nothing
+    const float4 a = seeds[2 * row];
+    const float4 b = seeds[2 * row + 1];
     lane_init(s, a, b, rng_seed, gid, seed_offset + gid);
     float c[CPAD];
 #pragma unroll
     for (int k = 0; k < CPAD; ++k) c[k] = 0.0f;
-    float4* line = out + (size_t)gid * p.n_steps;
-    line[0] = a;
-    while (s.n < p.n_steps && s.steps < p.max_steps) {
+    float4* line = out + row * p.n_steps;
+    if (own) line[0] = a;
+    bool live = own;
+    while (true) {
+        live = live && s.n < p.n_steps && s.steps < p.max_steps;
+        if (!__any_sync(0xffffffffu, live)) break;
         float qx, qy, qz;
-        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, s, c, qx, qy, qz);
-        if (r == 0) break;
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, live, s, c, qx, qy, qz);
+        live = r != 0;
         if (r == 2) {
             line[s.n] = make_float4(qx, qy, qz, 1.0f);
             s.n++;
         }
     }
-    lengths[gid] = s.n;
+    if (own) lengths[gid] = s.n;
 }
 
 // ------------------------------------------------------------- persistent
@@ -283,23 +287,20 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         }
         bool refill = false;
         bool slice_end = false;
+        float qx, qy, qz;
+        const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz, surface);
         if (live) {
-            bool done = s.n >= p.n_steps || s.steps >= p.max_steps;
+            bool done = r == 0;
             bool overflow = false;
-            if (!done) {
-                float qx, qy, qz;
-                const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, s, c, qx, qy, qz, surface);
-                if (r == 0) {
+            if (r == 2) {
+                if (emit_point(pp, chunk, fill, qx, qy, qz)) {
+                    s.n++;
+                    // a slice ends on a saved point: no test on the other steps
+                    if (SLICE && (s.n & pp.slice_mask) == 0u) slice_end = true;
+                } else {
                     done = true;
-                } else if (r == 2) {
-                    if (emit_point(pp, chunk, fill, qx, qy, qz)) {
-                        s.n++;
-                        // a slice ends on a saved point: no test on the other steps
-                        if (SLICE && (s.n & pp.slice_mask) == 0u) slice_end = true;
-                    } else {
-                        done = true;
-                        overflow = true;
-                    }
+                    overflow = true;
                 }
             }
             if (done) {
