@@ -694,6 +694,20 @@ static int tracker_pool(tg_tracker* t, uint64_t want_points)
     return TG_OK;
 }
 
+// Points the pool should hold for a run of at most `worst`: all of them where
+// that fits a third of the free memory, never fewer than `least`.  The free
+// memory is asked for only when the pool would have to grow: the query took
+// 0.1-0.3 ms of every call, and up to 10 ms with work in flight on the GPU.
+static uint64_t pool_points_wanted(const tg_tracker* t, uint64_t worst, uint64_t least)
+{
+    if (t->pool_points_request != 0) return t->pool_points_request;
+    if (t->pool != nullptr && (uint64_t)t->n_chunks * kChunkPoints >= worst) return worst;
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    const uint64_t budget = (uint64_t)(free_b / 3) / (3 * sizeof(float) + 1);
+    return std::min<uint64_t>(worst, std::max<uint64_t>(budget, least));
+}
+
 static int tracker_points(tg_tracker* t, uint64_t need, cudaStream_t s)
 {
     if (t->cap_points >= need && t->points != nullptr) return TG_OK;
@@ -772,14 +786,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
     // the pool is smaller and streamlines that run out are re-tracked in a
     // later wave (results depend only on the seed and its RNG stream).
     const uint64_t per_seed = ((uint64_t)n_steps + kChunkPoints - 1) / kChunkPoints * kChunkPoints;
-    uint64_t want = t->pool_points_request;
-    if (want == 0) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        const uint64_t budget = (uint64_t)(free_b / 3) / (3 * sizeof(float) + 1);
-        want = std::min<uint64_t>(per_seed * n_seeds, std::max<uint64_t>(budget, per_seed * 64));
-    }
-    st = tracker_pool(t, want);
+    st = tracker_pool(t, pool_points_wanted(t, per_seed * n_seeds, per_seed * 64));
     if (st != TG_OK) return st;
 
     PersistentParams pp;
@@ -1089,14 +1096,7 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
         TG_TRY(cudaMalloc(reinterpret_cast<void**>(&t->done_ids), n_total * sizeof(uint32_t)));
         t->cap_seeds = n_total;
     }
-    uint64_t want = t->pool_points_request;
-    if (want == 0) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        const uint64_t budget = (uint64_t)(free_b / 3) / (3 * sizeof(float) + 1);
-        want = std::min<uint64_t>(worst, std::max<uint64_t>(budget, (uint64_t)1 << 20));
-    }
-    int st = tracker_pool(t, want);
+    int st = tracker_pool(t, pool_points_wanted(t, worst, (uint64_t)1 << 20));
     if (st != TG_OK) return st;
 
     MultiParams mp;
