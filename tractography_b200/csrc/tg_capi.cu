@@ -814,7 +814,8 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
     const int block = persistent_block_size();
     int per_sm = persistent_blocks_per_sm(field->d, algorithm->algorithm, domain->d.kind);
     if (t->blocks_per_sm > 0 && (int)t->blocks_per_sm < per_sm) per_sm = (int)t->blocks_per_sm;
-    const int grid = sm_count() * per_sm;
+    const int sms = sm_count();
+    const int grid = sms * per_sm;
     const uint32_t rounds = t->compact_lanes > 0 ? t->compact_rounds : 0u;
     if (rounds > 0) {
         st = tracker_carry(t, kClassKinds, (size_t)grid * block);
@@ -857,6 +858,10 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
             TG_TRY(cudaMemcpyAsync(t->ids, wave_items.data(), n_items * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
         pp.item_ids = first_wave ? nullptr : t->ids;
         pp.n_items = n_items;
+        // later rounds of tail compaction resume as many streamlines as the
+        // device counts, and a round ends where warps are sparse: whole warps
+        pp.lanes = rounds > 0 ? 32u : spread_lanes(n_items, sms, per_sm);
+        const int wave_grid = rounds > 0 ? grid : spread_blocks(n_items, pp.lanes, sms, per_sm);
         pp.pool = t->pool;
         pp.chunk_next = t->chunk_next;
         pp.n_chunks = t->n_chunks;
@@ -881,7 +886,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
                 TG_TRY(cudaMemsetAsync(pp.ring.seq, 0, 2 * (size_t)pp.ring.capacity * sizeof(uint32_t), s));
                 TG_TRY(cudaMemsetAsync(pp.ring.ctl, 0, 2 * sizeof(unsigned int), s));
             }
-            TG_TRY(launch_track_persistent(field->d, pp, grid, block, s));
+            TG_TRY(launch_track_persistent(field->d, pp, wave_grid, block, s));
             t->launches += 1;
         }
         TG_TRY(cudaEventRecord(t->ev_stop, s));
@@ -1149,11 +1154,21 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
         // launch shapes and carry buffers first: no allocation while kernels run
         const uint32_t rounds = t->compact_lanes > 0 ? t->compact_rounds : 0u;
         std::vector<int> kgrid(kClassKinds, 0);
+        // the classes share the GPU: one spread for all of their streamlines
+        std::vector<int> kblocks(kClassKinds, 0);
+        int least = 32;
         for (int k : order) {
             if (members[k].empty()) continue;
-            int per_sm = class_blocks_per_sm(k);
-            if (t->blocks_per_sm > 0 && (int)t->blocks_per_sm < per_sm) per_sm = (int)t->blocks_per_sm;
-            kgrid[k] = sms * per_sm;
+            kblocks[k] = class_blocks_per_sm(k);
+            if (t->blocks_per_sm > 0 && (int)t->blocks_per_sm < kblocks[k]) kblocks[k] = (int)t->blocks_per_sm;
+            least = std::min(least, kblocks[k]);
+        }
+        const uint32_t lanes =
+            rounds > 0 ? 32u : spread_lanes(first_wave ? n_total : (uint64_t)wave_ids.size(), sms, least);
+        for (int k : order) {
+            if (members[k].empty()) continue;
+            const uint64_t n_k = first_wave ? lists[list_at[k] + 2 * members[k].size()] : (uint64_t)retry[k].size();
+            kgrid[k] = rounds > 0 ? sms * kblocks[k] : spread_blocks(n_k, lanes, sms, kblocks[k]);
             if (rounds > 0) {
                 st = tracker_carry(t, k, (size_t)kgrid[k] * 128);
                 if (st != TG_OK) return st;
@@ -1167,6 +1182,7 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
             cls.jobs = t->d_class_lists + list_at[k];
             cls.prefix = t->d_class_lists + list_at[k] + members[k].size();
             cls.counter = t->d_class_counters + k;
+            cls.lanes = lanes;
             if (first_wave) {
                 cls.n_items = members[k].empty() ? 0 : lists[list_at[k] + 2 * members[k].size()];
             } else {

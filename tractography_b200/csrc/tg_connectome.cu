@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
 
     // One loop iteration per step of every live lane; a lane whose track
     // ended finishes it and starts the next in the same iteration.
-    bool live = start();
+    bool live = (threadIdx.x & 31u) < q.lanes && start();
     while (__any_sync(0xffffffffu, live)) {
         bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
         __syncwarp();          // join locate()'s exits before the update (track_step)
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
 }
 
 template <int M, int L, int A, int D>
-cudaError_t run(const ConnectomeParams& q, cudaStream_t stream)
+cudaError_t run(ConnectomeParams q, cudaStream_t stream)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -125,8 +125,8 @@ cudaError_t run(const ConnectomeParams& q, cudaStream_t stream)
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, connectome_kernel<M, L, A, D>, 128, 0) != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
-    const uint64_t want = ((uint64_t)q.n_seeds + 127) / 128;
-    const int grid = (int)std::min<uint64_t>(want, (uint64_t)sms * per_sm);
+    q.lanes = spread_lanes(q.n_seeds, sms, per_sm);
+    const int grid = spread_blocks(q.n_seeds, q.lanes, sms, per_sm);
     connectome_kernel<M, L, A, D><<<grid, 128, 0, stream>>>(q);
     return cudaGetLastError();
 }

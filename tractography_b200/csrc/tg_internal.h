@@ -39,6 +39,36 @@ struct TrackRing {
     uint32_t lanes;      // lanes of the launch: claims in flight at most
 };
 
+// Lanes per warp that take streamlines in a launch of n of them (the lanes
+// from there up stay idle): n streamlines spread evenly over the SMs'
+// schedulers instead of filling the warps that reach the queue first, which
+// sat on a few SMs.  A launch that does not fill the GPU is bound by the
+// latency of its longest streamline's steps; a step is shorter where a warp
+// shares its scheduler with fewer others and where fewer lanes make it wait
+// for a new voxel.  So: as few warps per scheduler as hold n (k blocks of one
+// warp per scheduler and SM), then as few lanes per warp.  More warps of
+// fewer lanes measured slower (one B200, whole call): 10,000 Transport seeds
+// 6.0 / 6.1 / 6.4 / 6.7 ms with at least 1 / 2 / 3 / 4 warps per scheduler
+// (7.2 ms before the spread and before track_step's barrier), 30,011
+// counter-based SDE seeds at lmax 6 4.6 / 4.6 / 5.5 / 6.9 ms (8.7 ms).
+inline uint32_t spread_lanes(uint64_t n, int sms, int per_sm)
+{
+    const uint64_t warps = (uint64_t)sms * 4;          // one 128-lane block per SM
+    if (n >= warps * per_sm * 32) return 32;
+    const uint64_t k = (n + warps * 32 - 1) / (warps * 32);
+    const uint64_t lanes = k == 0 ? 1 : (n + warps * k - 1) / (warps * k);
+    return (uint32_t)(lanes < 1 ? 1 : lanes);
+}
+
+// Blocks of 128 lanes, `lanes` of each 32 in use, that n streamlines fill;
+// at most a full GPU.
+inline int spread_blocks(uint64_t n, uint32_t lanes, int sms, int per_sm)
+{
+    const uint64_t want = (n + 4ull * lanes - 1) / (4ull * lanes);
+    const uint64_t full = (uint64_t)sms * per_sm;
+    return (int)(want < 1 ? 1 : (want < full ? want : full));
+}
+
 constexpr int kChunkPoints = 32;   // points per output chunk (chunk = 32 x 12 B)
 
 // Device-resident image field (field.py:52-122): float32 coefficients,
@@ -109,6 +139,7 @@ struct PersistentParams {
     uint32_t n_seeds;
     const uint32_t* item_ids;     // nullable
     uint32_t n_items;
+    uint32_t lanes;               // lanes per warp that take streamlines (spread_lanes)
     uint32_t batch_size;
     const uint32_t* batch_rng_seeds;
     uint64_t seed_offset;         // Philox index base
@@ -169,6 +200,7 @@ struct ClassDev {
     const uint32_t* prefix;     // n_jobs + 1 prefix sums of their seed counts
     const uint32_t* item_ids;   // nullable: global seed indices to retry
     uint32_t n_items;
+    uint32_t lanes;             // lanes per warp that take streamlines (spread_lanes)
     unsigned long long* counter;
 };
 
@@ -211,6 +243,7 @@ struct TodParams {
     uint32_t n_steps;              // floor(maximum_streamline_length / step_size)
     float4 out_row0, out_row1, out_row2;   // output grid inverse affine rows
     uint32_t nx, ny, nz;
+    uint32_t lanes;                // lanes per warp that take tracks (spread_lanes; set by the launcher)
     float* coefficients;           // (nx, ny, nz, 45) float32, accumulated
     unsigned long long* steps;     // nullable: loop iterations that passed the domain and field tests
     unsigned long long* counter;   // next seed index (zeroed by the launcher)
@@ -230,6 +263,7 @@ struct ConnectomeParams {
     uint32_t n_seeds;
     uint32_t n_steps;
     float minimum_length;
+    uint32_t lanes;                // lanes per warp that take tracks (spread_lanes; set by the launcher)
     int32_t* rows;                 // 9 per seed, -1 when the track contributes nothing
     int32_t* columns;
     float* weights;

@@ -134,7 +134,7 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
         }
     };
 
-    bool live = fetch();
+    bool live = (threadIdx.x & 31u) < cls.lanes && fetch();
     while (true) {
         const unsigned active = __ballot_sync(0xffffffffu, live);
         if (active == 0u) break;

@@ -61,8 +61,8 @@ uint32_t* g_scratch_addr[kMaxDevices] = {};
 template <int MODEL, int LMAX, int ALGO>
 __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams p, const float4* __restrict__ seeds,
                                                                      uint32_t n_seeds, uint32_t batch_size,
-                                                                     uint64_t seed_offset, uint32_t* scratch,
-                                                                     float4* __restrict__ out,
+                                                                     uint64_t seed_offset, uint32_t lanes,
+                                                                     uint32_t* scratch, float4* __restrict__ out,
                                                                      uint32_t* __restrict__ lengths)
 {
     constexpr int CPAD = ModelShape<MODEL, LMAX>::CPAD;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
         line[0] = a;
         return true;
     };
-    bool live = fetch();
+    bool live = (threadIdx.x & 31u) < lanes && fetch();
     while (__any_sync(0xffffffffu, live)) {
         float qx, qy, qz;
         const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
@@ -115,9 +115,11 @@ cudaError_t launch_variant(const TrackParams& p, const float4* seeds, uint32_t n
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, track_persistent_dense_kernel<M, L, A>, 128, 0);
     if (e != cudaSuccess) return e;
-    const int grid = (sms > 0 ? sms : 1) * (blocks > 0 ? blocks : 1);
-    track_persistent_dense_kernel<M, L, A><<<grid, 128, 0, stream>>>(p, seeds, n, batch_size, seed_offset, scratch,
-                                                                      out, lengths);
+    sms = sms > 0 ? sms : 1;
+    blocks = blocks > 0 ? blocks : 1;
+    const uint32_t lanes = spread_lanes(n, sms, blocks);
+    track_persistent_dense_kernel<M, L, A><<<spread_blocks(n, lanes, sms, blocks), 128, 0, stream>>>(
+        p, seeds, n, batch_size, seed_offset, lanes, scratch, out, lengths);
     return cudaGetLastError();
 }
 

@@ -108,6 +108,7 @@ struct ServeParams {
     ServePool P;
     const LaneCarry* carry_in;
     uint32_t n_carry;
+    uint32_t lanes;              // lanes per warp that take streamlines (spread_lanes)
     LaneCarry* carry_out;
     unsigned int* carry_out_count;
     const uint32_t* seg_slot;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         return true;
     };
 
-    bool live = fetch();
+    bool live = (threadIdx.x & 31u) < sp.lanes && fetch();
     while (true) {
         const unsigned active = __ballot_sync(0xffffffffu, live);
         if (active == 0u) break;
@@ -944,6 +945,11 @@ int tg_server_poll(tg_server* S, uint64_t* finished_ids, uint32_t capacity, uint
     if (any) {
         const double t0 = now_s();
         int grid[kServeKinds] = {};
+        // one spread for the streamlines of all kinds (spread_lanes)
+        int least = 32;
+        for (int k = 0; k < kServeKinds; ++k)
+            if (n_new[k] != 0 || S->carry_n[k] != 0) least = std::min(least, kind_blocks(S, k));
+        const uint32_t lanes = spread_lanes(offered, S->sms, least);
         for (int k = 0; k < kServeKinds; ++k) {
             if (n_new[k] == 0 && S->carry_n[k] == 0) continue;
             // every kind is launched with as many blocks as its work fills,
@@ -952,8 +958,8 @@ int tg_server_poll(tg_server* S, uint64_t* finished_ids, uint32_t capacity, uint
             // split would leave them idle until the deadline).  At least one
             // lane per carried streamline (it resumes in the lane's first fetch).
             const int full = S->sms * kind_blocks(S, k);
-            const int need = (int)((S->carry_n[k] + 127) / 128);
-            const int work = (int)std::min<uint64_t>((uint64_t)full, (n_new[k] + S->carry_n[k] + 127) / 128);
+            const int need = (int)((S->carry_n[k] + 4 * lanes - 1) / (4 * lanes));
+            const int work = spread_blocks(n_new[k] + S->carry_n[k], lanes, S->sms, kind_blocks(S, k));
             grid[k] = std::max(1, std::max(need, work));
             st = ensure_carry(S, k, (size_t)full * 128);
             if (st != TG_OK) return st;
@@ -1007,6 +1013,7 @@ int tg_server_poll(tg_server* S, uint64_t* finished_ids, uint32_t capacity, uint
             sp.P = S->P;
             sp.carry_in = S->carry[k][S->carry_cur[k]];
             sp.n_carry = S->carry_n[k];
+            sp.lanes = lanes;
             sp.carry_out = S->carry[k][S->carry_cur[k] ^ 1];
             sp.carry_out_count = S->d_carry_count + k;
             sp.seg_slot = S->d_segs + at[k][0];

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
     // ended flushes it and starts the next in the same iteration, so lanes
     // stay busy while the queue lasts (a loop per track would hold finished
     // lanes until the warp's longest track ends).
-    bool live = start();
+    bool live = (threadIdx.x & 31u) < q.lanes && start();
     while (__any_sync(0xffffffffu, live)) {
         bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
         __syncwarp();          // join locate()'s exits before the update (track_step)
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
 }
 
 template <int M, int L, int A, int D>
-cudaError_t run_tod(const TodParams& q, cudaStream_t stream)
+cudaError_t run_tod(TodParams q, cudaStream_t stream)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -136,8 +136,8 @@ cudaError_t run_tod(const TodParams& q, cudaStream_t stream)
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tod_kernel<M, L, A, D>, kTodThreads, 0) !=
             cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const uint64_t want = ((uint64_t)q.n_seeds + kTodThreads - 1) / kTodThreads;
-    const int grid = (int)std::min<uint64_t>(want, (uint64_t)sms * per_sm);
+    q.lanes = spread_lanes(q.n_seeds, sms, per_sm);
+    const int grid = spread_blocks(q.n_seeds, q.lanes, sms, per_sm);
     tod_kernel<M, L, A, D><<<grid, kTodThreads, 0, stream>>>(q);
     return cudaGetLastError();
 }

@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         }
     };
 
-    live = fetch();
+    const bool takes = (threadIdx.x & 31u) < pp.lanes;
+    live = takes && fetch();
     while (true) {
         const unsigned active = __ballot_sync(0xffffffffu, live);
         if (active == 0u) break;
