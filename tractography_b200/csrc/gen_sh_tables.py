@@ -23,10 +23,11 @@ Outputs (committed next to this script):
   tg_sh_eval.cuh  -- CUDA device code: straight-line evaluation for
                      LMAX in {0, 2, 4, 6, 8} performing, in the same order,
                      the operations the table-driven CPU evaluation performs.
-  tg_sh_fold.h    -- plain C / CUDA: the fold of a coefficient vector into
-                     per-order polynomials in u (tgsh_fold, double sums).
-  tg_sh_folded.cuh -- CUDA device code: straight-line evaluation of the
-                     folded form (what the tracking kernels run per step).
+  tg_sh_fold.h    -- plain C: the fold of a coefficient vector into per-order
+                     polynomials in u (tgsh_fold, double sums).
+  tg_sh_folded.cuh -- CUDA device code: the same fold in straight line, and
+                     the straight-line evaluation of the folded form (what
+                     the tracking kernels run per step).
 """
 
 from fractions import Fraction
@@ -338,13 +339,8 @@ def write_fold_header():
         "#ifndef TG_SH_FOLD_H",
         "#define TG_SH_FOLD_H",
         "",
-        "#if defined(__CUDACC__)",
-        "#define TGSH_FN __device__ __forceinline__",
-        "#define TGSH_TABLE __device__ __constant__",
-        "#else",
         "#define TGSH_FN static inline",
         "#define TGSH_TABLE static const",
-        "#endif",
         "",
     ]
     offsets = []
@@ -405,13 +401,19 @@ def write_fold_header():
 
 
 def write_fold_eval():
-    """Straight-line CUDA evaluation of the folded form, in the operation order of
-    the oracle's block loop."""
+    """Straight-line CUDA fold (tgsh_fold's sums) and evaluation of the folded form,
+    in the operation order of the oracle's block loop."""
     out = [
         "/* Generated by gen_sh_tables.py -- do not edit. */",
-        "/* Value, d/dtheta and (d/dphi)/sin(theta) of the real symmetric SH model",
-        " * from folded coefficients (tg_sh_fold.h): per order m and part, S(u) and",
-        " * S'(u) by one Horner pass, then A = x^p S and dA/dx. */",
+        "/* The fold of a voxel's SH coefficients (tgsh_fold's sums), and the value,",
+        " * d/dtheta and (d/dphi)/sin(theta) of the real symmetric SH model from it: per",
+        " * order m and part, S(u) and S'(u) by one Horner pass, then A = x^p S and dA/dx.",
+        " * Written for scalar instructions: with cosine and sine part of an order in",
+        " * register pairs (tg_f32x2.cuh) it took 147 instructions instead of 182 but, at",
+        " * 96 registers, 40 to 150 bytes of spills, and the paired multiply-adds hold the",
+        " * arithmetic pipe for two cycles each: 593 ms against 558 ms for 100k SDE seeds.",
+        " * Each order's trigonometric factors and powers stand right before their block:",
+        " * all of them up front took 570 ms where this order takes 540 ms. */",
         "#ifndef TG_SH_FOLDED_CUH",
         "#define TG_SH_FOLDED_CUH",
         "",
@@ -419,6 +421,12 @@ def write_fold_eval():
         "",
     ]
     for lmax in range(0, LMAX + 1, 2):
+        sums = {}
+        for dst, src, r in fold_terms(lmax)[0]:
+            sums[dst] = f"({sums.get(dst, '0.0')} + (double)c[{src}] * {hexd(r)})"
+        out += [f"template <> __device__ __forceinline__ void sh_fold<{lmax}>(const float* c, float* a)", "{"]
+        out += [f"    a[{dst}] = (float){sums[dst]};" for dst in sorted(sums)]
+        out += ["}", ""]
         blocks, n = fold_blocks(lmax)
         out += [
             f"template <> __device__ __forceinline__ void sh_eval_folded<{lmax}>(",
@@ -435,18 +443,21 @@ def write_fold_eval():
         ]
         if lmax >= 1:
             out.append("    const float cm1 = cp, sm1 = sp;")
-        for m in range(2, lmax + 1):
-            out.append(f"    const float cm{m} = fmaf(tc, cm{m-1}, -cm{m-2});")
-            out.append(f"    const float sm{m} = fmaf(tc, sm{m-1}, -sm{m-2});")
         out.append("    const float stp0 = 1.0f;")
         out.append("    (void)stp0;")
-        for k in range(1, lmax + 2):
-            out.append(f"    const float stp{k} = stp{k-1} * st;")
         out.append("    float val = 0.0f, dth = 0.0f, dph = 0.0f;")
         by_m = {}
         for blk in blocks:
             by_m.setdefault(blk[0], []).append(blk)
+        powers = 0
         for m in sorted(by_m):
+            # each order's cosine, sine and powers of sin(theta) right before its block
+            if m >= 2:
+                out.append(f"    const float cm{m} = fmaf(tc, cm{m-1}, -cm{m-2});")
+                out.append(f"    const float sm{m} = fmaf(tc, sm{m-1}, -sm{m-2});")
+            while powers < min(m + 1, lmax + 1):
+                powers += 1
+                out.append(f"    const float stp{powers} = stp{powers-1} * st;")
             out.append("    {")
             names = ["A", "B"]
             has_deriv = False

@@ -162,7 +162,7 @@ __global__ void cost_update(const float* in, float* out, int n, AlgoParams a)
     float raw[45], c[45];
     for (int k = 0; k < 45; ++k) raw[k] = in[(i * 7 + k) % n] * 0.05f;
     raw[0] = 0.3f;
-    tgsh_fold(8, raw, c);
+    sh_fold<8>(raw, c);
     RngState rng;
     rng.mwc = rng_init(7u, (uint32_t)i);
     rng.index = (uint64_t)i;

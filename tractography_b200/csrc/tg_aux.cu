@@ -188,7 +188,7 @@ __global__ void field_evaluate_kernel(Grid g, const float* __restrict__ field, u
     for (uint32_t j = 0; j < C; ++j) out[(size_t)i * C + j] = k >= 0 ? field[k * cpad + j] : 0.0f;
 }
 
-// The coefficients model_eval takes: SH coefficients folded (tgsh_fold),
+// The coefficients model_eval takes: SH coefficients folded (sh_fold),
 // tensor coefficients as they are.
 template <int MODEL, int LMAX, int CP>
 __device__ __forceinline__ void model_coefficients(const float (&raw)[CP], float (&c)[CP])
@@ -197,27 +197,39 @@ __device__ __forceinline__ void model_coefficients(const float (&raw)[CP], float
 #pragma unroll
         for (int k = 0; k < CP; ++k) c[k] = raw[k];
     } else {
-        tgsh_fold(LMAX, raw, c);
+        sh_fold<LMAX>(raw, c);
     }
 }
 
-// Folds a field's SH coefficients per voxel (cpad floats each, zero beyond
-// the band) for the tracking kernels.
-__global__ void fold_field_kernel(const float* __restrict__ raw, float* __restrict__ folded, uint64_t n_voxels,
-                                  uint32_t cpad, int lmax)
+// Folds a field's SH coefficients per voxel (CPAD floats each, zero beyond
+// the band) for the tracking kernels.  Bound by memory (8 CPAD bytes per
+// voxel); the fold is straight-line code on registers.
+template <int LMAX>
+__global__ void __launch_bounds__(128) fold_field_kernel(const float4* __restrict__ raw, float4* __restrict__ folded,
+                                                         uint64_t n_voxels)
 {
-    const int n = (lmax + 1) * (lmax + 2) / 2;
+    constexpr int N = n_coef_full(LMAX), CPAD = ModelShape<kModelSH, LMAX>::CPAD;
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n_voxels;
          v += (uint64_t)gridDim.x * blockDim.x) {
-        float c[48], a[48];
-        for (uint32_t k = 0; k < cpad; ++k) c[k] = raw[v * cpad + k];
-        tgsh_fold(lmax, c, a);
-        for (uint32_t k = 0; k < cpad; ++k) folded[v * cpad + k] = (int)k < n ? a[k] : 0.0f;
+        float c[CPAD], a[CPAD];
+#pragma unroll
+        for (int k = 0; k < CPAD / 4; ++k) {
+            const float4 q = __ldg(raw + v * (CPAD / 4) + k);
+            c[4 * k] = q.x;
+            c[4 * k + 1] = q.y;
+            c[4 * k + 2] = q.z;
+            c[4 * k + 3] = q.w;
+        }
+        sh_fold<LMAX>(c, a);
+#pragma unroll
+        for (int k = N; k < CPAD; ++k) a[k] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < CPAD / 4; ++k)
+            folded[v * (CPAD / 4) + k] = make_float4(a[4 * k], a[4 * k + 1], a[4 * k + 2], a[4 * k + 3]);
     }
 }
 
-cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels, uint32_t cpad, int lmax,
-                              cudaStream_t stream)
+cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels, int lmax, cudaStream_t stream)
 {
     if (n_voxels == 0) return cudaSuccess;
     int dev = 0, sms = 148;
@@ -226,7 +238,16 @@ cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels
     const int block = 128;
     uint64_t grid = (n_voxels + block - 1) / block;
     if (grid > (uint64_t)sms * 32) grid = (uint64_t)sms * 32;
-    fold_field_kernel<<<(int)grid, block, 0, stream>>>(raw, folded, n_voxels, cpad, lmax);
+    const float4* src = reinterpret_cast<const float4*>(raw);
+    float4* dst = reinterpret_cast<float4*>(folded);
+    switch (lmax) {
+    case 0: fold_field_kernel<0><<<(int)grid, block, 0, stream>>>(src, dst, n_voxels); break;
+    case 2: fold_field_kernel<2><<<(int)grid, block, 0, stream>>>(src, dst, n_voxels); break;
+    case 4: fold_field_kernel<4><<<(int)grid, block, 0, stream>>>(src, dst, n_voxels); break;
+    case 6: fold_field_kernel<6><<<(int)grid, block, 0, stream>>>(src, dst, n_voxels); break;
+    case 8: fold_field_kernel<8><<<(int)grid, block, 0, stream>>>(src, dst, n_voxels); break;
+    default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 

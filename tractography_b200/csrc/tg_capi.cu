@@ -360,7 +360,7 @@ int tg_field_create(int32_t model, const float* values, uint32_t nx, uint32_t ny
     // the trackers' copy: SH coefficients folded per voxel, tensors as given
     if (e == cudaSuccess && model == TG_MODEL_SH) {
         e = cudaMalloc(reinterpret_cast<void**>(&f->d.folded), f->d.bytes);
-        if (e == cudaSuccess) e = launch_fold_field(f->d.data, f->d.folded, nvox, f->d.cpad, f->d.lmax, s);
+        if (e == cudaSuccess) e = launch_fold_field(f->d.data, f->d.folded, nvox, f->d.lmax, s);
     } else if (e == cudaSuccess) {
         f->d.folded = f->d.data;
     }

@@ -34,13 +34,14 @@ __device__ __forceinline__ void sh_eval(const float* c, float ct, float st, floa
 template <int LMAX>
 __device__ __forceinline__ void sh_basis(float ct, float st, float cp, float sp, float* Y);
 template <int LMAX>
+__device__ __forceinline__ void sh_fold(const float* c, float* a);
+template <int LMAX>
 __device__ __forceinline__ void sh_eval_folded(const float* a, float ct, float st, float cp, float sp,
                                                float* val, float* dth, float* dph);
 
 }  // namespace tg
 
 #include "tg_sh_eval.cuh"
-#include "tg_sh_fold.h"
 #include "tg_sh_folded.cuh"
 
 namespace tg {
@@ -221,7 +222,7 @@ __device__ __forceinline__ float softmax(float x, float k)
     return x;
 }
 
-// local.py:91-120 from folded coefficients (tgsh_fold): the field the
+// local.py:91-120 from folded coefficients (sh_fold): the field the
 // trackers read is folded once per voxel when it is created.
 template <int LMAX>
 __device__ __forceinline__ ModelValue sh_model(const float* folded, const Frame& f)

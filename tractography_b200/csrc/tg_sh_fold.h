@@ -5,13 +5,8 @@
 #ifndef TG_SH_FOLD_H
 #define TG_SH_FOLD_H
 
-#if defined(__CUDACC__)
-#define TGSH_FN __device__ __forceinline__
-#define TGSH_TABLE __device__ __constant__
-#else
 #define TGSH_FN static inline
 #define TGSH_TABLE static const
-#endif
 
 #define TGSH_NTERMS 175
 /* per band limit 0, 2, .., 8: first term, term count, folded length */
