@@ -165,10 +165,8 @@ __global__ void cost_update(const float* in, float* out, int n, AlgoParams a)
     sh_fold<8>(raw, c);
     RngState rng;
     rng.mwc = rng_init(7u, (uint32_t)i);
-    rng.index = (uint64_t)i;
-    rng.step = 0u;
     float ox = 0.0f, oy = 0.6f, oz = 0.8f;
-    for (int r = 0; r < REPS; ++r) update_orientation<kModelSH, 8, ALGO>(a, c, ox, oy, oz, rng);
+    for (int r = 0; r < REPS; ++r) update_orientation<kModelSH, 8, ALGO>(a, c, ox, oy, oz, rng, (uint32_t)r);
     out[i] = ox + oy + oz;
 }
 

@@ -282,12 +282,9 @@ __global__ void update_orientation_kernel(AlgoParams a, uint32_t rng_seed, uint6
 #pragma unroll
     for (int k = 0; k < CP; ++k) raw[k] = (uint32_t)k < n_params ? params[(size_t)i * n_params + k] : 0.0f;
     model_coefficients<MODEL, LMAX, CP>(raw, c);
-    RngState rng;
-    rng.mwc = rng_init(rng_seed, i);
-    rng.index = seed_offset + i;
-    rng.step = 0u;
+    RngState rng = rng_state(a, rng_init(rng_seed, i), seed_offset + i);
     float4 v = o[i];
-    update_orientation<MODEL, LMAX, ALGO>(a, c, v.x, v.y, v.z, rng);
+    update_orientation<MODEL, LMAX, ALGO>(a, c, v.x, v.y, v.z, rng, 0u);
     out[i] = make_float4(v.x, v.y, v.z, 0.0f);
 }
 

@@ -49,6 +49,7 @@ namespace tg {
 
 constexpr int kDomainImage = 0;
 constexpr int kDomainMesh = 1;
+constexpr int kDomainSame = 2;    // kernels: a mask on the field's own grid
 
 // Cell word: distance (low 8 bits) | leaf list offset in 16-byte units.
 constexpr uint32_t kNoLeafList = 0xFFFFFFu;

@@ -63,8 +63,8 @@ struct tg_tracker {
     std::vector<uint32_t> h_done;
     std::vector<uint32_t> h_retry;
     // multi-job runs: one stream per code path, job and class tables
-    cudaStream_t class_stream[kClassKinds] = {};
-    cudaEvent_t class_done[kClassKinds] = {};
+    cudaStream_t class_stream[kJobKinds] = {};
+    cudaEvent_t class_done[kJobKinds] = {};
     cudaEvent_t ev_fork = nullptr;
     JobDev* d_jobs = nullptr;
     size_t cap_jobs = 0;
@@ -74,7 +74,7 @@ struct tg_tracker {
     size_t cap_class_lists = 0;
     unsigned long long* d_class_counters = nullptr;
     // launch shape and tail compaction (tg_tracker_set_tuning); slot
-    // kClassKinds holds the single-job tracker's carry buffers
+    // kJobKinds holds the single-job tracker's carry buffers
     uint32_t blocks_per_sm = 0;        // 0: the occupancy maximum
     uint32_t compact_lanes = 0;        // 0: no compaction (measured faster by default)
     uint32_t compact_rounds = 4;
@@ -87,8 +87,8 @@ struct tg_tracker {
     size_t cap_ring_flags = 0;
     unsigned int* ring_ctl = nullptr;  // head, tail, fault, spare
     size_t cap_ring_ctl = 0;
-    LaneCarry* carry[kClassKinds + 1][2] = {};
-    size_t carry_cap[kClassKinds + 1] = {};
+    LaneCarry* carry[kJobKinds + 1][2] = {};
+    size_t carry_cap[kJobKinds + 1] = {};
     unsigned int* carry_count = nullptr;   // 2 per slot
     // statistics of the last run
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -594,7 +594,7 @@ int tg_tracker_destroy(tg_tracker* t)
     cudaFree(t->ring_ctl);
     if (t->ev_start) cudaEventDestroy(t->ev_start);
     if (t->ev_stop) cudaEventDestroy(t->ev_stop);
-    for (int k = 0; k < kClassKinds; ++k) {
+    for (int k = 0; k < kJobKinds; ++k) {
         if (t->class_stream[k]) cudaStreamDestroy(t->class_stream[k]);
         if (t->class_done[k]) cudaEventDestroy(t->class_done[k]);
     }
@@ -603,7 +603,7 @@ int tg_tracker_destroy(tg_tracker* t)
     cudaFree(t->d_job_base);
     cudaFree(t->d_class_lists);
     cudaFree(t->d_class_counters);
-    for (int k = 0; k <= kClassKinds; ++k) {
+    for (int k = 0; k <= kJobKinds; ++k) {
         cudaFree(t->carry[k][0]);
         cudaFree(t->carry[k][1]);
     }
@@ -664,7 +664,7 @@ int tg_tracker_stats(const tg_tracker* t, float* kernel_ms, uint32_t* waves, uin
 static int tracker_carry(tg_tracker* t, int slot, size_t lanes)
 {
     if (t->carry_count == nullptr) {
-        TG_TRY(cudaMalloc(reinterpret_cast<void**>(&t->carry_count), 2 * (kClassKinds + 1) * sizeof(unsigned int)));
+        TG_TRY(cudaMalloc(reinterpret_cast<void**>(&t->carry_count), 2 * (kJobKinds + 1) * sizeof(unsigned int)));
     }
     if (t->carry_cap[slot] >= lanes && t->carry[slot][0] != nullptr) return TG_OK;
     cudaFree(t->carry[slot][0]);
@@ -812,13 +812,13 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
     }
 
     const int block = persistent_block_size();
-    int per_sm = persistent_blocks_per_sm(field->d, algorithm->algorithm, domain->d.kind);
+    int per_sm = persistent_blocks_per_sm(field->d, algorithm->algorithm, domain_form(tp));
     if (t->blocks_per_sm > 0 && (int)t->blocks_per_sm < per_sm) per_sm = (int)t->blocks_per_sm;
     const int sms = sm_count();
     const int grid = sms * per_sm;
     const uint32_t rounds = t->compact_lanes > 0 ? t->compact_rounds : 0u;
     if (rounds > 0) {
-        st = tracker_carry(t, kClassKinds, (size_t)grid * block);
+        st = tracker_carry(t, kJobKinds, (size_t)grid * block);
         if (st != TG_OK) return st;
     }
     // slicing only where a streamline can outlast a slice
@@ -844,7 +844,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
         while ((uint64_t)slice_points * 2 <= points && slice_points < (1u << 30)) slice_points *= 2;
         pp.slice_mask = slice_points - 1u;
     }
-    unsigned int* ccount = t->carry_count + 2 * kClassKinds;
+    unsigned int* ccount = t->carry_count + 2 * kJobKinds;
 
     t->h_len.resize(n_seeds);
     TG_TRY(cudaMemsetAsync(t->counters + 1, 0, sizeof(unsigned long long), s));
@@ -875,9 +875,9 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
         // by sparse warps of the previous round; the last round compacts no more
         for (uint32_t r = 0; r <= rounds; ++r) {
             TG_TRY(cudaMemsetAsync(t->counters, 0, sizeof(unsigned long long), s));
-            pp.carry_in = r == 0 ? nullptr : t->carry[kClassKinds][(r - 1) & 1];
+            pp.carry_in = r == 0 ? nullptr : t->carry[kJobKinds][(r - 1) & 1];
             pp.carry_in_count = r == 0 ? nullptr : ccount + ((r - 1) & 1);
-            pp.carry_out = r < rounds ? t->carry[kClassKinds][r & 1] : nullptr;
+            pp.carry_out = r < rounds ? t->carry[kJobKinds][r & 1] : nullptr;
             pp.carry_out_count = ccount + (r & 1);
             pp.compact_lanes = t->compact_lanes;
             if (r < rounds) TG_TRY(cudaMemsetAsync(ccount + (r & 1), 0, sizeof(unsigned int), s));
@@ -1018,7 +1018,7 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
         table[j].n_seeds = J.n_seeds;
         table[j].batch_size = J.batch_size > 0 ? J.batch_size : 1;
         table[j].seed_offset = J.algorithm.seed_offset;
-        kind[j] = class_kind(J.field->d.model, J.field->d.lmax, J.algorithm.algorithm);
+        kind[j] = job_kind(class_kind(J.field->d.model, J.field->d.lmax, J.algorithm.algorithm), tp.same_grid != 0);
         job_base[j] = (uint32_t)n_total;
         rng_base[j] = (uint32_t)n_batches_total;
         n_total += J.n_seeds;
@@ -1053,12 +1053,12 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
     TG_TRY(cudaMemcpyAsync(t->d_job_base, job_base.data(), (n_jobs + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
 
     // Classes: jobs grouped by code path, longest point budget first.
-    std::vector<std::vector<uint32_t>> members(kClassKinds);
+    std::vector<std::vector<uint32_t>> members(kJobKinds);
     for (uint32_t j = 0; j < n_jobs; ++j)
         if (jobs[j].n_seeds > 0) members[kind[j]].push_back(j);
     std::vector<uint32_t> lists;            // per class: jobs then prefix (n + 1)
-    std::vector<size_t> list_at(kClassKinds, 0);
-    for (int k = 0; k < kClassKinds; ++k) {
+    std::vector<size_t> list_at(kJobKinds, 0);
+    for (int k = 0; k < kJobKinds; ++k) {
         auto& m = members[k];
         std::stable_sort(m.begin(), m.end(), [&](uint32_t a, uint32_t b) { return jobs[a].n_steps > jobs[b].n_steps; });
         list_at[k] = lists.size();
@@ -1073,9 +1073,9 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
     TG_TRY(ensure(&t->d_class_lists, &t->cap_class_lists, lists.size()));
     TG_TRY(cudaMemcpyAsync(t->d_class_lists, lists.data(), lists.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     if (t->d_class_counters == nullptr)
-        TG_TRY(cudaMalloc(reinterpret_cast<void**>(&t->d_class_counters), kClassKinds * sizeof(unsigned long long)));
+        TG_TRY(cudaMalloc(reinterpret_cast<void**>(&t->d_class_counters), kJobKinds * sizeof(unsigned long long)));
     if (t->ev_fork == nullptr) TG_TRY(cudaEventCreateWithFlags(&t->ev_fork, cudaEventDisableTiming));
-    for (int k = 0; k < kClassKinds; ++k) {
+    for (int k = 0; k < kJobKinds; ++k) {
         if (members[k].empty() || t->class_stream[k] != nullptr) continue;
         TG_TRY(cudaStreamCreateWithFlags(&t->class_stream[k], cudaStreamNonBlocking));
         TG_TRY(cudaEventCreateWithFlags(&t->class_done[k], cudaEventDisableTiming));
@@ -1121,14 +1121,14 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
     uint64_t total = 0;
     bool first_wave = true;
     int stalls = 0;
-    std::vector<std::vector<uint32_t>> retry(kClassKinds);
+    std::vector<std::vector<uint32_t>> retry(kJobKinds);
     std::vector<uint32_t> wave_ids;
     while (true) {
         // per class: its item source for this wave
-        std::vector<size_t> retry_at(kClassKinds, 0);
+        std::vector<size_t> retry_at(kJobKinds, 0);
         uint64_t wave_items = 0;
         wave_ids.clear();
-        for (int k = 0; k < kClassKinds; ++k) {
+        for (int k = 0; k < kJobKinds; ++k) {
             retry_at[k] = wave_ids.size();
             if (!first_wave) wave_ids.insert(wave_ids.end(), retry[k].begin(), retry[k].end());
         }
@@ -1139,23 +1139,23 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
         mp.pool = t->pool;
         mp.chunk_next = t->chunk_next;
         mp.n_chunks = t->n_chunks;
-        TG_TRY(cudaMemsetAsync(t->d_class_counters, 0, kClassKinds * sizeof(unsigned long long), s));
+        TG_TRY(cudaMemsetAsync(t->d_class_counters, 0, kJobKinds * sizeof(unsigned long long), s));
         TG_TRY(cudaMemsetAsync(t->chunk_counter, 0, sizeof(unsigned int), s));
         TG_TRY(cudaEventRecord(t->ev_start, s));
         TG_TRY(cudaEventRecord(t->ev_fork, s));
         std::vector<int> launched;
         // classes with the most point budget first
         std::vector<int> order;
-        for (int k = 0; k < kClassKinds; ++k) order.push_back(k);
-        std::vector<uint64_t> budget(kClassKinds, 0);
-        for (int k = 0; k < kClassKinds; ++k)
+        for (int k = 0; k < kJobKinds; ++k) order.push_back(k);
+        std::vector<uint64_t> budget(kJobKinds, 0);
+        for (int k = 0; k < kJobKinds; ++k)
             for (uint32_t j : members[k]) budget[k] += (uint64_t)jobs[j].n_seeds * jobs[j].n_steps;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return budget[a] > budget[b]; });
         // launch shapes and carry buffers first: no allocation while kernels run
         const uint32_t rounds = t->compact_lanes > 0 ? t->compact_rounds : 0u;
-        std::vector<int> kgrid(kClassKinds, 0);
+        std::vector<int> kgrid(kJobKinds, 0);
         // the classes share the GPU: one spread for all of their streamlines
-        std::vector<int> kblocks(kClassKinds, 0);
+        std::vector<int> kblocks(kJobKinds, 0);
         int least = 32;
         for (int k : order) {
             if (members[k].empty()) continue;
@@ -1252,7 +1252,7 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
 
         // collect finished streamlines, queue the others for the next wave
         t->h_done.clear();
-        std::vector<std::vector<uint32_t>> next(kClassKinds);
+        std::vector<std::vector<uint32_t>> next(kJobKinds);
         auto visit = [&](uint32_t g, int k) {
             const uint32_t L = t->h_len[g];
             if (L & kOverflowBit) {

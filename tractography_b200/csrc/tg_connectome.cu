@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
         float px, py, pz, ox, oy, oz;
         sample_boundary(q.vertices, q.triangles, q.cumulative, q.n_triangles, st, px, py, pz, ox, oy, oz, &start_tri,
                         start_w);
-        lane_init(s, make_float4(px, py, pz, 1.0f), make_float4(ox, oy, oz, 0.0f), 0u, 0u, q.seed_offset + gid);
-        s.rng.mwc = st;
+        lane_init(s, p.algo, make_float4(px, py, pz, 1.0f), make_float4(ox, oy, oz, 0.0f), 0u, 0u, 0ull);
+        s.rng = rng_state(p.algo, st, q.seed_offset + gid);
         qx = px;
         qy = py;
         qz = pz;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
         bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
         __syncwarp();          // join locate()'s exits before the update (track_step)
         if (go) {
-            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng);
+            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
             s.steps += 1u;
             const float len = sqrtf(s.ox * s.ox + s.oy * s.oy + s.oz * s.oz);
             if (!(isfinite(s.ox) && isfinite(s.oy) && isfinite(s.oz)) || len < 0.5f) {
@@ -134,7 +134,10 @@ cudaError_t run(ConnectomeParams q, cudaStream_t stream)
 template <int M, int L, int A>
 cudaError_t run_domain(const ConnectomeParams& q, cudaStream_t stream)
 {
-    return q.t.domain_kind == kDomainMesh ? run<M, L, A, kDomainMesh>(q, stream) : run<M, L, A, kDomainImage>(q, stream);
+    const int form = domain_form(q.t);
+    return form == kDomainMesh   ? run<M, L, A, kDomainMesh>(q, stream)
+           : form == kDomainSame ? run<M, L, A, kDomainSame>(q, stream)
+                                 : run<M, L, A, kDomainImage>(q, stream);
 }
 
 }  // namespace

@@ -115,7 +115,7 @@ struct TrackParams {
     Grid fgrid;
     const float* field;
     uint32_t cpad;
-    int same_grid;           // domain and field inverse affines/dims identical
+    int same_grid;           // mask: domain and field inverse affines/dims identical
     int algorithm;           // kTransport or kDiffusion
     AlgoParams algo;
     float save_at;
@@ -126,6 +126,13 @@ struct TrackParams {
     // inputs the host accepts; it only guarantees that every lane ends.
     uint32_t max_steps;
 };
+
+// Which form of the domain test a launch compiles in: kDomainMesh,
+// kDomainSame or kDomainImage.
+inline int domain_form(const TrackParams& p)
+{
+    return p.domain_kind == kDomainMesh ? kDomainMesh : (p.same_grid ? kDomainSame : kDomainImage);
+}
 
 // Batched persistent launch over work items 0..n_items-1; item k tracks
 // seed item_ids[k] (or k when item_ids is null).  Seed i belongs to batch
@@ -193,6 +200,10 @@ enum ClassKind : int {
     kSH0T, kSH0D, kSH2T, kSH2D, kSH4T, kSH4D, kSH6T, kSH6D, kSH8T, kSH8D, kDTIT, kDTID, kClassKinds
 };
 
+// The code paths of a multi-job run: per class, masks on the field's grid (odd)
+// and on their own (even).
+constexpr int kJobKinds = 2 * kClassKinds;
+
 struct ClassDev {
     int kind;
     uint32_t n_jobs;
@@ -229,6 +240,7 @@ struct MultiParams {
 cudaError_t launch_track_class(const MultiParams& mp, const ClassDev& cls, int grid, cudaStream_t stream);
 int class_blocks_per_sm(int kind);
 int class_kind(int model, int lmax, int algorithm);
+int job_kind(int class_kind, bool same_grid);   // 0 .. kJobKinds - 1
 
 // Track orientation distribution (tg_tod.cu, tracking.py:181-385).
 struct TodParams {
@@ -339,7 +351,7 @@ cudaError_t launch_rng_streams(int which, uint32_t s0, uint32_t s1, uint32_t n, 
 
 int lmax_for(uint32_t n_params);
 int persistent_block_size();
-int persistent_blocks_per_sm(const FieldDev& f, int algorithm, int domain_kind);
+int persistent_blocks_per_sm(const FieldDev& f, int algorithm, int form);
 
 }  // namespace tg
 

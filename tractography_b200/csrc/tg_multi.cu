@@ -26,6 +26,8 @@ int class_kind(int model, int lmax, int algorithm)
     return base + (algorithm == kTransport ? 0 : 1);
 }
 
+int job_kind(int class_kind, bool same_grid) { return 2 * class_kind + (same_grid ? 1 : 0); }
+
 namespace {
 
 __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t v)
@@ -74,7 +76,7 @@ __device__ __forceinline__ bool m_emit(const MultiParams& mp, int32_t& chunk, ui
 // wavefront per distinct job per load.
 constexpr int kSharedJobs = 48;
 
-template <int MODEL, int LMAX, int ALGO>
+template <int MODEL, int LMAX, int ALGO, int DOM>
 __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp, const ClassDev& cls,
                                                           const TrackParams* shared_t, uint32_t n_shared)
 {
@@ -120,7 +122,7 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
             const float4 a = J->seeds[2 * (size_t)i];
             const float4 b = J->seeds[2 * (size_t)i + 1];
             const uint32_t batch = i / J->batch_size;
-            lane_init(s, a, b, mp.batch_rng_seeds[J->rng_base + batch], i - batch * J->batch_size,
+            lane_init(s, P->algo, a, b, mp.batch_rng_seeds[J->rng_base + batch], i - batch * J->batch_size,
                       J->seed_offset + i);
             if (!m_chunk_alloc(mp, chunk)) {
                 mp.first_chunk[g] = -1;
@@ -145,7 +147,7 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
         }
         float qx, qy, qz;
         const bool go = live && s.n < P->n_steps && s.steps < P->max_steps;
-        const int r = track_step<MODEL, LMAX, ALGO, CPAD>(*P, go, s, c, qx, qy, qz);
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(*P, go, s, c, qx, qy, qz);
         if (!live) continue;
         bool done = r == 0;
         bool overflow = false;
@@ -166,7 +168,7 @@ __device__ __forceinline__ unsigned long long drain_class(const MultiParams& mp,
     return steps_total;
 }
 
-template <int MODEL, int LMAX, int ALGO>
+template <int MODEL, int LMAX, int ALGO, int DOM>
 __global__ void __launch_bounds__(128, 5) track_class_kernel(const MultiParams mp, const ClassDev cls)
 {
     extern __shared__ uint4 shared_raw[];
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(128, 5) track_class_kernel(const MultiParams m
             reinterpret_cast<const uint32_t*>(&mp.jobs[cls.jobs[q]].t)[o];
     }
     __syncthreads();
-    const unsigned long long steps = drain_class<MODEL, LMAX, ALGO>(mp, cls, table, n_shared);
+    const unsigned long long steps = drain_class<MODEL, LMAX, ALGO, DOM>(mp, cls, table, n_shared);
     if (steps != 0) atomicAdd(mp.steps_done, steps);
 }
 
@@ -190,42 +192,46 @@ size_t class_shared_bytes(uint32_t n_jobs)
     return (size_t)n * sizeof(TrackParams);
 }
 
-template <int M, int L, int A>
+template <int M, int L, int A, int D>
 struct ClassLaunch {
     static cudaError_t run(const MultiParams& mp, const ClassDev& cls, int grid, cudaStream_t stream)
     {
-        track_class_kernel<M, L, A><<<grid, 128, class_shared_bytes(cls.n_jobs), stream>>>(mp, cls);
+        track_class_kernel<M, L, A, D><<<grid, 128, class_shared_bytes(cls.n_jobs), stream>>>(mp, cls);
         return cudaGetLastError();
     }
 };
 
-template <int M, int L, int A>
+template <int M, int L, int A, int D>
 struct ClassOccupancy {
     static cudaError_t run(int* blocks)
     {
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, track_class_kernel<M, L, A>, 128,
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, track_class_kernel<M, L, A, D>, 128,
                                                              class_shared_bytes(kSharedJobs));
     }
 };
 
-template <template <int, int, int> class Fn, typename... Args>
+template <template <int, int, int, int> class Fn, typename... Args>
 cudaError_t class_dispatch(int kind, Args&&... args)
 {
-    switch (kind) {
-    case kSH0T: return Fn<kModelSH, 0, kTransport>::run(args...);
-    case kSH0D: return Fn<kModelSH, 0, kDiffusion>::run(args...);
-    case kSH2T: return Fn<kModelSH, 2, kTransport>::run(args...);
-    case kSH2D: return Fn<kModelSH, 2, kDiffusion>::run(args...);
-    case kSH4T: return Fn<kModelSH, 4, kTransport>::run(args...);
-    case kSH4D: return Fn<kModelSH, 4, kDiffusion>::run(args...);
-    case kSH6T: return Fn<kModelSH, 6, kTransport>::run(args...);
-    case kSH6D: return Fn<kModelSH, 6, kDiffusion>::run(args...);
-    case kSH8T: return Fn<kModelSH, 8, kTransport>::run(args...);
-    case kSH8D: return Fn<kModelSH, 8, kDiffusion>::run(args...);
-    case kDTIT: return Fn<kModelDTI, 0, kTransport>::run(args...);
-    case kDTID: return Fn<kModelDTI, 0, kDiffusion>::run(args...);
+    const bool same = (kind & 1) != 0;
+#define TG_CLASS(K, M, L, A) \
+    case K: return same ? Fn<M, L, A, kDomainSame>::run(args...) : Fn<M, L, A, kDomainImage>::run(args...);
+    switch (kind >> 1) {
+        TG_CLASS(kSH0T, kModelSH, 0, kTransport)
+        TG_CLASS(kSH0D, kModelSH, 0, kDiffusion)
+        TG_CLASS(kSH2T, kModelSH, 2, kTransport)
+        TG_CLASS(kSH2D, kModelSH, 2, kDiffusion)
+        TG_CLASS(kSH4T, kModelSH, 4, kTransport)
+        TG_CLASS(kSH4D, kModelSH, 4, kDiffusion)
+        TG_CLASS(kSH6T, kModelSH, 6, kTransport)
+        TG_CLASS(kSH6D, kModelSH, 6, kDiffusion)
+        TG_CLASS(kSH8T, kModelSH, 8, kTransport)
+        TG_CLASS(kSH8D, kModelSH, 8, kDiffusion)
+        TG_CLASS(kDTIT, kModelDTI, 0, kTransport)
+        TG_CLASS(kDTID, kModelDTI, 0, kDiffusion)
     default: return cudaErrorInvalidValue;
     }
+#undef TG_CLASS
 }
 
 }  // namespace

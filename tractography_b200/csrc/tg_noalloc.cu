@@ -58,7 +58,7 @@ constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
 uint32_t* g_scratch_addr[kMaxDevices] = {};
 
-template <int MODEL, int LMAX, int ALGO>
+template <int MODEL, int LMAX, int ALGO, int DOM>
 __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams p, const float4* __restrict__ seeds,
                                                                      uint32_t n_seeds, uint32_t batch_size,
                                                                      uint64_t seed_offset, uint32_t lanes,
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
         const uint32_t local = item - batch * batch_size;
         const float4 a = seeds[2 * (size_t)item];
         const float4 b = seeds[2 * (size_t)item + 1];
-        lane_init(s, a, b, batch_seeds[batch], local, seed_offset + item);
+        lane_init(s, p.algo, a, b, batch_seeds[batch], local, seed_offset + item);
         line = out + (size_t)item * p.n_steps;
         line[0] = a;
         return true;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
     while (__any_sync(0xffffffffu, live)) {
         float qx, qy, qz;
         const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
-        const int r = track_step<MODEL, LMAX, ALGO, CPAD>(p, go, s, c, qx, qy, qz);
+        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz);
         if (!live) continue;
         if (r == 2) {
             line[s.n] = make_float4(qx, qy, qz, 1.0f);
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
     }
 }
 
-template <int M, int L, int A>
+template <int M, int L, int A, int D>
 cudaError_t launch_variant(const TrackParams& p, const float4* seeds, uint32_t n, uint32_t batch_size,
                            uint64_t seed_offset, uint32_t* scratch, float4* out, uint32_t* lengths,
                            cudaStream_t stream)
@@ -113,12 +113,12 @@ cudaError_t launch_variant(const TrackParams& p, const float4* seeds, uint32_t n
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, track_persistent_dense_kernel<M, L, A>, 128, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, track_persistent_dense_kernel<M, L, A, D>, 128, 0);
     if (e != cudaSuccess) return e;
     sms = sms > 0 ? sms : 1;
     blocks = blocks > 0 ? blocks : 1;
     const uint32_t lanes = spread_lanes(n, sms, blocks);
-    track_persistent_dense_kernel<M, L, A><<<spread_blocks(n, lanes, sms, blocks), 128, 0, stream>>>(
+    track_persistent_dense_kernel<M, L, A, D><<<spread_blocks(n, lanes, sms, blocks), 128, 0, stream>>>(
         p, seeds, n, batch_size, seed_offset, lanes, scratch, out, lengths);
     return cudaGetLastError();
 }
@@ -129,7 +129,9 @@ cudaError_t launch(int model, int lmax, int algo, const TrackParams& p, const fl
 {
 #define TG_NA_CASE(M, L, A)                                                                      \
     if (model == M && (M == kModelDTI || lmax == L) && algo == A)                                \
-        return launch_variant<M, L, A>(p, seeds, n, batch_size, seed_offset, scratch, out, lengths, s);
+        return p.same_grid                                                                       \
+                   ? launch_variant<M, L, A, kDomainSame>(p, seeds, n, batch_size, seed_offset, scratch, out, lengths, s)  \
+                   : launch_variant<M, L, A, kDomainImage>(p, seeds, n, batch_size, seed_offset, scratch, out, lengths, s);
     TG_NA_CASE(kModelSH, 0, kTransport) TG_NA_CASE(kModelSH, 0, kDiffusion)
     TG_NA_CASE(kModelSH, 2, kTransport) TG_NA_CASE(kModelSH, 2, kDiffusion)
     TG_NA_CASE(kModelSH, 4, kTransport) TG_NA_CASE(kModelSH, 4, kDiffusion)

@@ -65,7 +65,7 @@ int track_params_from_handles(const tg_algorithm* a, const tg_domain* d, const t
 
 namespace {
 
-constexpr int kServeKinds = 2 * kClassKinds;     // code path x domain kind
+constexpr int kServeKinds = 3 * kClassKinds;     // code path x domain kind
 
 struct ServeJob {
     TrackParams t;
@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             const float4 a = J->seeds[2 * (size_t)item];
             const float4 b = J->seeds[2 * (size_t)item + 1];
             const uint32_t batch = item / J->batch_size;
-            lane_init(s, a, b, J->batch_rng_seeds[batch], item - batch * J->batch_size, J->seed_offset + item);
+            lane_init(s, J->t.algo, a, b, J->batch_rng_seeds[batch], item - batch * J->batch_size,
+                      J->seed_offset + item);
             if (DOM == kDomainMesh && J->seed_inside != nullptr) s.seed_state = J->seed_inside[item] ? 1u : 2u;
             atomicAdd(J->counts, 1u);
             chunk = -1;
@@ -317,11 +318,12 @@ struct ServeOccupancy {
 template <template <int, int, int, int> class Fn, typename... Args>
 cudaError_t serve_dispatch(int kind, Args&&... args)
 {
-    const int cls = kind >> 1;
-    const bool mesh = (kind & 1) != 0;
+    const int cls = kind / 3, form = kind % 3;
 #define TG_SERVE(K, M, L, A)                                                                          \
     case K:                                                                                          \
-        return mesh ? Fn<M, L, A, kDomainMesh>::run(args...) : Fn<M, L, A, kDomainImage>::run(args...);
+        return form == kDomainMesh   ? Fn<M, L, A, kDomainMesh>::run(args...)                        \
+               : form == kDomainSame ? Fn<M, L, A, kDomainSame>::run(args...)                        \
+                                     : Fn<M, L, A, kDomainImage>::run(args...);
     switch (cls) {
         TG_SERVE(kSH0T, kModelSH, 0, kTransport)
         TG_SERVE(kSH0D, kModelSH, 0, kDiffusion)
@@ -877,7 +879,7 @@ int tg_server_submit(tg_server* S, const tg_job* job, uint64_t* request_id)
         return sfail(TG_ERR_POOL_EXHAUSTED, "the server's point pool cannot hold one streamline of this request");
     ServeRequest* r = new ServeRequest();
     r->id = S->next_id++;
-    r->kind = 2 * class_kind(model, lmax, job->algorithm.algorithm) + (tp.domain_kind == kDomainMesh ? 1 : 0);
+    r->kind = 3 * class_kind(model, lmax, job->algorithm.algorithm) + domain_form(tp);
     r->job = *job;
     r->tp = tp;
     const uint32_t n = job->n_seeds;

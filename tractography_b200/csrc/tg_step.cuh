@@ -32,13 +32,11 @@ struct Lane {
     float time;
     uint32_t n;
     RngState rng;
-    // Voxel cache of the last domain test and field gather; while it holds,
-    // the mask bit (inside) and the coefficients in registers are still
-    // valid, so the voxel rounding, bounds tests, index arithmetic and loads
-    // are skipped.  Domain and field on one grid: the open interval
-    // (dv, fv) per axis in which both voxels are unchanged.  Otherwise (and
-    // for closed surfaces, fv only): the rounded voxel coordinates of the
-    // domain test (dv) and the field gather (fv).  NaN forces an evaluation.
+    // Voxel cache: the rounded voxel coordinates of the last domain test (dv;
+    // only where domain and field have different grids) and field gather
+    // (fv); while they hold, the mask bit (inside) and the coefficients in
+    // registers are still valid, so the voxel rounding, bounds tests, index
+    // arithmetic and loads are skipped.  NaN forces an evaluation.
     float dvx, dvy, dvz;
     float fvx, fvy, fvz;
     uint32_t steps;
@@ -49,8 +47,24 @@ struct Lane {
     uint32_t seed_state;
 };
 
-// DOM selects the domain test: the image mask (domain.py:358-382), or a
-// closed surface, where the seed must be inside and every later point must
+// The coefficients of field voxel (fx, fy, fz) (field.py:88-114).
+template <int CPAD>
+__device__ __forceinline__ void load_voxel(const TrackParams& p, float fx, float fy, float fz, float (&c)[CPAD])
+{
+    const int64_t fv = ((int64_t)(int32_t)fx * p.fgrid.ny + (int32_t)fy) * p.fgrid.nz + (int32_t)fz;
+    const float4* src = reinterpret_cast<const float4*>(p.field) + fv * (CPAD / 4);
+#pragma unroll
+    for (int k = 0; k < CPAD / 4; ++k) {
+        const float4 v = __ldg(src + k);
+        c[4 * k] = v.x;
+        c[4 * k + 1] = v.y;
+        c[4 * k + 2] = v.z;
+        c[4 * k + 3] = v.w;
+    }
+}
+
+// DOM selects the domain test: the image mask (domain.py:358-382; kDomainSame
+// when it lies on the field's grid, kDomainImage otherwise), or a closed surface, where the seed must be inside and every later point must
 // be reached by a segment from the previous one that does not hit the
 // surface (the found flag of bvh.cl:83-131).
 //
@@ -77,52 +91,43 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
         ax = dot4(p.fgrid.row0, s.px, s.py, s.pz, 1.0f);
         ay = dot4(p.fgrid.row1, s.px, s.py, s.pz, 1.0f);
         az = dot4(p.fgrid.row2, s.px, s.py, s.pz, 1.0f);
-    } else {
+    } else if constexpr (DOM == kDomainSame) {
         // domain.py:358-382 and field.py:88-114 share the voxel-space point
         // when both images have the same grid (the default of tg.tractogram).
         ax = dot4(p.dgrid.row0, s.px, s.py, s.pz, 1.0f);
         ay = dot4(p.dgrid.row1, s.px, s.py, s.pz, 1.0f);
         az = dot4(p.dgrid.row2, s.px, s.py, s.pz, 1.0f);
-        if (p.same_grid) {
-            // For a voxel f and f - 0.5 < a < f + 0.5 (open), rint(a) = f and
-            // floor(fl(a + 0.5)) = f: the sum lies in [f, f + 1) after rounding
-            // (f is representable and a + 0.5 < f + 1 rounds to at most a
-            // value below f + 1 for |a| < 2^22).  So six comparisons with the
-            // cached interval certify both voxels unchanged.
-            if (ax > s.dvx && ax < s.fvx && ay > s.dvy && ay < s.fvy && az > s.dvz && az < s.fvz) return true;
-            const float vx = floorf(ax + 0.5f), vy = floorf(ay + 0.5f), vz = floorf(az + 0.5f);
-            const float fx = rintf(ax), fy = rintf(ay), fz = rintf(az);
-            if (!(vx >= 0.0f && vx < (float)p.dgrid.nx && vy >= 0.0f && vy < (float)p.dgrid.ny && vz >= 0.0f &&
-                  vz < (float)p.dgrid.nz))
-                return false;
-            if (!(fx >= 0.0f && fx < (float)p.fgrid.nx && fy >= 0.0f && fy < (float)p.fgrid.ny && fz >= 0.0f &&
-                  fz < (float)p.fgrid.nz))
-                return false;
-            const int64_t k = ((int64_t)(int32_t)vx * p.dgrid.ny + (int32_t)vy) * p.dgrid.nz + (int32_t)vz;
-            const uint8_t inside = __ldg(p.mask + k);
-            const int64_t fv = ((int64_t)(int32_t)fx * p.fgrid.ny + (int32_t)fy) * p.fgrid.nz + (int32_t)fz;
-            const float4* src = reinterpret_cast<const float4*>(p.field) + fv * (CPAD / 4);
-#pragma unroll
-            for (int k4 = 0; k4 < CPAD / 4; ++k4) {
-                const float4 v = __ldg(src + k4);
-                c[4 * k4] = v.x;
-                c[4 * k4 + 1] = v.y;
-                c[4 * k4 + 2] = v.z;
-                c[4 * k4 + 3] = v.w;
-            }
-            if (inside == 0) return false;
-            // a point on a voxel face (a = f + 0.5 exactly) has different
-            // domain and field voxels: leave the cache invalid
-            const bool tie = vx != fx || vy != fy || vz != fz;
-            const float nan = __int_as_float(0x7fc00000);
-            s.dvx = tie ? nan : fx - 0.5f;
-            s.dvy = tie ? nan : fy - 0.5f;
-            s.dvz = tie ? nan : fz - 0.5f;
-            s.fvx = tie ? nan : fx + 0.5f;
-            s.fvy = tie ? nan : fy + 0.5f;
-            s.fvz = tie ? nan : fz + 0.5f;
-            return true;
-        }
+        // For a voxel f and f - 0.5 < a < f + 0.5 (open), rint(a) = f and
+        // floor(fl(a + 0.5)) = f: the sum lies in [f, f + 1) after rounding
+        // (f is representable and a + 0.5 < f + 1 rounds to at most a
+        // value below f + 1 for |a| < 2^22).  So |a - f| < 0.5 for the cached
+        // voxel certifies both unchanged: the difference is exact in that
+        // interval (f = 0, or a and f within a factor of two), and outside
+        // it rounds to no less than 0.5.
+        if (fabsf(ax - s.fvx) < 0.5f && fabsf(ay - s.fvy) < 0.5f && fabsf(az - s.fvz) < 0.5f) return true;
+        const float vx = floorf(ax + 0.5f), vy = floorf(ay + 0.5f), vz = floorf(az + 0.5f);
+        const float fx = rintf(ax), fy = rintf(ay), fz = rintf(az);
+        if (!(vx >= 0.0f && vx < (float)p.dgrid.nx && vy >= 0.0f && vy < (float)p.dgrid.ny && vz >= 0.0f &&
+              vz < (float)p.dgrid.nz))
+            return false;
+        if (!(fx >= 0.0f && fx < (float)p.fgrid.nx && fy >= 0.0f && fy < (float)p.fgrid.ny && fz >= 0.0f &&
+              fz < (float)p.fgrid.nz))
+            return false;
+        const int64_t k = ((int64_t)(int32_t)vx * p.dgrid.ny + (int32_t)vy) * p.dgrid.nz + (int32_t)vz;
+        const uint8_t inside = __ldg(p.mask + k);
+        load_voxel(p, fx, fy, fz, c);
+        if (inside == 0) return false;
+        // a point on a voxel face (a = f + 0.5 exactly) has different
+        // domain and field voxels: leave the cache invalid
+        const bool tie = vx != fx || vy != fy || vz != fz;
+        s.fvx = tie ? __int_as_float(0x7fc00000) : fx;
+        s.fvy = fy;
+        s.fvz = fz;
+        return true;
+    } else {
+        ax = dot4(p.dgrid.row0, s.px, s.py, s.pz, 1.0f);
+        ay = dot4(p.dgrid.row1, s.px, s.py, s.pz, 1.0f);
+        az = dot4(p.dgrid.row2, s.px, s.py, s.pz, 1.0f);
         const float vx = floorf(ax + 0.5f), vy = floorf(ay + 0.5f), vz = floorf(az + 0.5f);
         const float bx = dot4(p.fgrid.row0, s.px, s.py, s.pz, 1.0f);
         const float by = dot4(p.fgrid.row1, s.px, s.py, s.pz, 1.0f);
@@ -146,18 +151,7 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
             const int64_t k = ((int64_t)(int32_t)vx * p.dgrid.ny + (int32_t)vy) * p.dgrid.nz + (int32_t)vz;
             inside = __ldg(p.mask + k);
         }
-        if (fchange) {
-            const int64_t fv = ((int64_t)(int32_t)fx * p.fgrid.ny + (int32_t)fy) * p.fgrid.nz + (int32_t)fz;
-            const float4* src = reinterpret_cast<const float4*>(p.field) + fv * (CPAD / 4);
-#pragma unroll
-            for (int k = 0; k < CPAD / 4; ++k) {
-                const float4 v = __ldg(src + k);
-                c[4 * k] = v.x;
-                c[4 * k + 1] = v.y;
-                c[4 * k + 2] = v.z;
-                c[4 * k + 3] = v.w;
-            }
-        }
+        if (fchange) load_voxel(p, fx, fy, fz, c);
         if (inside == 0) return false;
         if (dchange) {
             s.dvx = vx;
@@ -177,16 +171,7 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
         if (!(fx >= 0.0f && fx < (float)p.fgrid.nx && fy >= 0.0f && fy < (float)p.fgrid.ny &&
               fz >= 0.0f && fz < (float)p.fgrid.nz))
             return false;
-        const int64_t fv = ((int64_t)(int32_t)fx * p.fgrid.ny + (int32_t)fy) * p.fgrid.nz + (int32_t)fz;
-        const float4* src = reinterpret_cast<const float4*>(p.field) + fv * (CPAD / 4);
-#pragma unroll
-        for (int k = 0; k < CPAD / 4; ++k) {
-            const float4 v = __ldg(src + k);
-            c[4 * k] = v.x;
-            c[4 * k + 1] = v.y;
-            c[4 * k + 2] = v.z;
-            c[4 * k + 3] = v.w;
-        }
+        load_voxel(p, fx, fy, fz, c);
         s.fvx = fx;
         s.fvy = fy;
         s.fvz = fz;
@@ -213,7 +198,7 @@ __device__ __forceinline__ int track_step(const TrackParams& p, bool go, Lane& s
     if (go) go = locate<MODEL, LMAX, CPAD, DOM>(p, s, c, surface);
     __syncwarp();
     if (!go) return 0;
-    update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng);
+    update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
     s.steps += 1u;
 
     const float step = p.algo.step_size;
@@ -284,8 +269,7 @@ struct __align__(16) LaneCarry {
     float ox, oy, oz, lx;
     float ly, lz;
     uint32_t n, steps;
-    uint32_t mwc_x, mwc_c, rng_step, item;
-    uint64_t rng_index;
+    uint32_t mwc_x, mwc_c, item;
     int32_t chunk;
     uint32_t fill;
     uint32_t job;            // job slot (multi-request serving); 0 otherwise
@@ -304,11 +288,9 @@ __device__ __forceinline__ void lane_save(LaneCarry* dst, const Lane& s, uint32_
     c.ly = s.ly; c.lz = s.lz; c.n = s.n; c.steps = s.steps;
     c.item = item;
     if (RNG) {
-        c.mwc_x = s.rng.mwc.x; c.mwc_c = s.rng.mwc.c; c.rng_step = s.rng.step;
-        c.rng_index = s.rng.index;
+        c.mwc_x = s.rng.mwc.x; c.mwc_c = s.rng.mwc.c;
     } else {
-        c.mwc_x = 0u; c.mwc_c = 0u; c.rng_step = 0u;
-        c.rng_index = 0ull;
+        c.mwc_x = 0u; c.mwc_c = 0u;
     }
     c.chunk = chunk;
     c.fill = fill;
@@ -324,8 +306,7 @@ __device__ __forceinline__ void lane_restore(Lane& s, const LaneCarry& c, uint32
     s.ly = c.ly; s.lz = c.lz; s.n = c.n; s.steps = c.steps;
     item = c.item;
     if (RNG) {
-        s.rng.mwc.x = c.mwc_x; s.rng.mwc.c = c.mwc_c; s.rng.step = c.rng_step;
-        s.rng.index = c.rng_index;
+        s.rng.mwc.x = c.mwc_x; s.rng.mwc.c = c.mwc_c;
     }
     s.dvx = s.dvy = s.dvz = __int_as_float(0x7fc00000);
     s.fvx = s.fvy = s.fvz = __int_as_float(0x7fc00000);
@@ -352,16 +333,14 @@ __device__ __forceinline__ bool warp_should_compact(unsigned active, uint32_t co
     return active != 0xffffffffu && (uint32_t)__popc(active) <= compact_lanes;
 }
 
-__device__ __forceinline__ void lane_init(Lane& s, float4 a, float4 b, uint32_t rng_seed,
+__device__ __forceinline__ void lane_init(Lane& s, const AlgoParams& algo, float4 a, float4 b, uint32_t rng_seed,
                                           uint32_t stream_id, uint64_t index)
 {
     s.px = a.x; s.py = a.y; s.pz = a.z;
     s.ox = b.x; s.oy = b.y; s.oz = b.z;
     s.time = 0.0f;
     s.n = 1;
-    s.rng.mwc = rng_init(rng_seed, stream_id);
-    s.rng.index = index;
-    s.rng.step = 0u;
+    s.rng = rng_state(algo, rng_init(rng_seed, stream_id), index);
     s.dvx = s.dvy = s.dvz = __int_as_float(0x7fc00000);
     s.fvx = s.fvy = s.fvz = __int_as_float(0x7fc00000);
     s.steps = 0u;

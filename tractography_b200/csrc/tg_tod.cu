@@ -63,8 +63,8 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
         Mwc st = rng_init(q.rng_seed, gid);
         float px, py, pz, ox, oy, oz;
         sample_boundary(q.vertices, q.triangles, q.cumulative, q.n_triangles, st, px, py, pz, ox, oy, oz);
-        lane_init(s, make_float4(px, py, pz, 1.0f), make_float4(ox, oy, oz, 0.0f), 0u, 0u, q.seed_offset + gid);
-        s.rng.mwc = st;
+        lane_init(s, p.algo, make_float4(px, py, pz, 1.0f), make_float4(ox, oy, oz, 0.0f), 0u, 0u, 0ull);
+        s.rng = rng_state(p.algo, st, q.seed_offset + gid);
         prev_x = prev_y = prev_z = -1;
         step = 0;
         return true;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
                 tod_flush(q.coefficients, acc, tid, prev_x, prev_y, prev_z, q);
                 prev_x = prev_y = prev_z = -1;
             }
-            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng);
+            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
             s.steps += 1u;
             // tracking.py:343: stop on a non-finite or degenerate orientation
             const float len = sqrtf(s.ox * s.ox + s.oy * s.oy + s.oz * s.oz);
@@ -145,8 +145,10 @@ cudaError_t run_tod(TodParams q, cudaStream_t stream)
 template <int M, int L, int A>
 cudaError_t run_tod_domain(const TodParams& q, cudaStream_t stream)
 {
-    return q.t.domain_kind == kDomainMesh ? run_tod<M, L, A, kDomainMesh>(q, stream)
-                                          : run_tod<M, L, A, kDomainImage>(q, stream);
+    const int form = domain_form(q.t);
+    return form == kDomainMesh   ? run_tod<M, L, A, kDomainMesh>(q, stream)
+           : form == kDomainSame ? run_tod<M, L, A, kDomainSame>(q, stream)
+                                 : run_tod<M, L, A, kDomainImage>(q, stream);
 }
 
 }  // namespace

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128) track_dense_kernel(TrackParams p, const f
     const size_t row = own ? gid : 0;      // lanes past the end keep their warp whole and track nothing
     const float4 a = seeds[2 * row];
     const float4 b = seeds[2 * row + 1];
-    lane_init(s, a, b, rng_seed, gid, seed_offset + gid);
+    lane_init(s, p.algo, a, b, rng_seed, gid, seed_offset + gid);
     float c[CPAD];
 #pragma unroll
     for (int k = 0; k < CPAD; ++k) c[k] = 0.0f;
@@ -221,7 +221,6 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
     uint32_t fill = 0;
     uint32_t item = 0;
     bool live = false;
-    unsigned long long steps_total = 0;
 
     const unsigned long long n_items = pp.carry_in != nullptr ? *pp.carry_in_count : pp.n_items;
 
@@ -242,7 +241,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             const float4 b = pp.seeds[2 * (size_t)item + 1];
             const uint32_t batch = item / pp.batch_size;
             const uint32_t local = item - batch * pp.batch_size;
-            lane_init(s, a, b, pp.batch_rng_seeds[batch], local, pp.seed_offset + item);
+            lane_init(s, p.algo, a, b, pp.batch_rng_seeds[batch], local, pp.seed_offset + item);
             if (DOM == kDomainMesh && pp.seed_inside != nullptr) s.seed_state = pp.seed_inside[item] ? 1u : 2u;
             if (!chunk_alloc(pp, chunk)) {
                 pp.first_chunk[item] = -1;
@@ -306,7 +305,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             }
             if (done) {
                 pp.lengths[item] = overflow ? (s.n | kOverflowBit) : s.n;
-                if (!overflow) steps_total += s.steps;
+                if (!overflow && pp.steps_done != nullptr) atomicAdd(pp.steps_done, (unsigned long long)s.steps);
                 refill = true;
             } else if (SLICE && slice_end && work_waiting(pp, n_items)) {
                 ring_push<ALGO != kTransport>(pp.ring, s, item, chunk, fill);
@@ -319,7 +318,6 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         if (SLICE) __syncwarp();
         if (refill) live = fetch();
     }
-    if (pp.steps_done != nullptr && steps_total != 0) atomicAdd(pp.steps_done, steps_total);
 }
 
 // ----------------------------------------------------------------- gather
@@ -361,8 +359,9 @@ cudaError_t dispatch(int model, int lmax, int algo, int dom, Args&&... args)
 {
 #define TG_CASE(M, L, A)                                                                     \
     if (model == M && (M == kModelDTI || lmax == L) && algo == A)                            \
-        return dom == kDomainMesh ? Fn<M, L, A, kDomainMesh>::run(args...)                   \
-                                  : Fn<M, L, A, kDomainImage>::run(args...);
+        return dom == kDomainMesh   ? Fn<M, L, A, kDomainMesh>::run(args...)                 \
+               : dom == kDomainSame ? Fn<M, L, A, kDomainSame>::run(args...)                 \
+                                    : Fn<M, L, A, kDomainImage>::run(args...);
     TG_CASE(kModelSH, 0, kTransport) TG_CASE(kModelSH, 0, kDiffusion)
     TG_CASE(kModelSH, 2, kTransport) TG_CASE(kModelSH, 2, kDiffusion)
     TG_CASE(kModelSH, 4, kTransport) TG_CASE(kModelSH, 4, kDiffusion)
@@ -415,10 +414,10 @@ int lmax_for(uint32_t n_params)
 
 int persistent_block_size() { return 128; }
 
-int persistent_blocks_per_sm(const FieldDev& f, int algorithm, int domain_kind)
+int persistent_blocks_per_sm(const FieldDev& f, int algorithm, int form)
 {
     int blocks = 0;
-    if (dispatch<PersistentOccupancy>(f.model, f.lmax, algorithm, domain_kind, &blocks) != cudaSuccess ||
+    if (dispatch<PersistentOccupancy>(f.model, f.lmax, algorithm, form, &blocks) != cudaSuccess ||
         blocks < 1)
         blocks = 1;
     return blocks;
@@ -429,7 +428,7 @@ cudaError_t launch_track_dense(const FieldDev& f, const TrackParams& p, const fl
                                uint32_t* lengths, cudaStream_t stream)
 {
     if (n_seeds == 0) return cudaSuccess;
-    return dispatch<DenseLaunch>(f.model, f.lmax, p.algorithm, p.domain_kind, p, seeds, n_seeds, rng_seed,
+    return dispatch<DenseLaunch>(f.model, f.lmax, p.algorithm, domain_form(p), p, seeds, n_seeds, rng_seed,
                                  seed_offset,
                                  out, lengths, stream);
 }
@@ -438,7 +437,7 @@ cudaError_t launch_track_persistent(const FieldDev& f, const PersistentParams& p
                                     cudaStream_t stream)
 {
     if (p.n_items == 0) return cudaSuccess;
-    return dispatch<PersistentLaunch>(f.model, f.lmax, p.t.algorithm, p.t.domain_kind, p, grid, block, stream);
+    return dispatch<PersistentLaunch>(f.model, f.lmax, p.t.algorithm, domain_form(p.t), p, grid, block, stream);
 }
 
 cudaError_t launch_gather(const float* pool, const int32_t* chunk_next, const int32_t* first_chunk,
