@@ -248,14 +248,16 @@ def write_cuda(entries):
             out.append("    float cm1 = cp, sm1 = sp;")
         else:
             out.append("    (void)tc; (void)st; (void)sp;")
-        for m in range(2, lmax + 1):
-            out.append(f"    const float cm{m} = fmaf(tc, cm{m-1}, -cm{m-2});")
-            out.append(f"    const float sm{m} = fmaf(tc, sm{m-1}, -sm{m-2});")
         if lmax >= 1:
             out.append("    float stp0 = 1.0f; (void)stp0;")
-            for k in range(1, lmax + 1):
-                out.append(f"    const float stp{k} = stp{k-1} * st;")
+        order = 0
         for (l, m, parity, r, rp) in [e for e in entries if e[0] <= lmax]:
+            while order < m:     # an order's cosine, sine and power of sin(theta) right before its terms
+                order += 1
+                if order >= 2:
+                    out.append(f"    const float cm{order} = fmaf(tc, cm{order-1}, -cm{order-2});")
+                    out.append(f"    const float sm{order} = fmaf(tc, sm{order-1}, -sm{order-2});")
+                out.append(f"    const float stp{order} = stp{order-1} * st;")
             ip = l * (l + 1) // 2 + m
             im = l * (l + 1) // 2 - m
             out.append("    {")

@@ -93,8 +93,7 @@ __global__ void __launch_bounds__(128) connectome_kernel(const ConnectomeParams 
         if (go) {
             update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
             s.steps += 1u;
-            const float len = sqrtf(s.ox * s.ox + s.oy * s.oy + s.oz * s.oz);
-            if (!(isfinite(s.ox) && isfinite(s.oy) && isfinite(s.oz)) || len < 0.5f) {
+            if (degenerate(s.ox, s.oy, s.oz)) {
                 go = false;
             } else {
                 qx = s.px;

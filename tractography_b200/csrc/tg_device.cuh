@@ -401,12 +401,12 @@ __device__ __forceinline__ void exps2(float& ox, float& oy, float& oz, float tx,
     oz = fmaf(tz, k, c * oz);
 }
 
-// step: updates made before this one (the counter-based stream's counter).
+// f: the frame of (ox, oy, oz); step: updates made before this one (the
+// counter-based stream's counter).
 template <int MODEL, int LMAX, int ALGO>
-__device__ __forceinline__ void update_orientation(const AlgoParams& a, const float* c,
+__device__ __forceinline__ void update_orientation(const AlgoParams& a, const float* c, const Frame& f,
                                                    float& ox, float& oy, float& oz, RngState& rng, uint32_t step)
 {
-    const Frame f = frame_of(ox, oy, oz);
     const ModelValue mv = model_eval<MODEL, LMAX>(c, ox, oy, oz, f);
     const float etx = f.ct * f.cp, ety = f.ct * f.sp, etz = -f.st;
     const float epx = -f.sp, epy = f.cp;
@@ -438,6 +438,23 @@ __device__ __forceinline__ void update_orientation(const AlgoParams& a, const fl
         tz = fmaf(a.scale_noise, nz, a.scale_drift * dz);
     }
     exps2(ox, oy, oz, tx, ty, tz);
+}
+
+template <int MODEL, int LMAX, int ALGO>
+__device__ __forceinline__ void update_orientation(const AlgoParams& a, const float* c,
+                                                   float& ox, float& oy, float& oz, RngState& rng, uint32_t step)
+{
+    update_orientation<MODEL, LMAX, ALGO>(a, c, frame_of(ox, oy, oz), ox, oy, oz, rng, step);
+}
+
+// tracking.py:343: a track stops on a non-finite orientation or one
+// shorter than 0.5.  sqrt is correctly rounded and monotonic, so len < 0.5 is
+// len^2 < 0.25, and a finite len^2 has finite components.
+__device__ __forceinline__ bool degenerate(float x, float y, float z)
+{
+    const float len2 = x * x + y * y + z * z;
+    if (len2 >= 0.25f && len2 < __int_as_float(0x7f800000)) return false;
+    return !(isfinite(x) && isfinite(y) && isfinite(z)) || len2 < 0.25f;
 }
 
 // ----------------------------------------------------- domain / field

@@ -949,11 +949,7 @@ template <> __device__ __forceinline__ void sh_basis<2>(
     (void)u;
     const float cm0 = 1.0f, sm0 = 0.0f; (void)cm0; (void)sm0;
     float cm1 = cp, sm1 = sp;
-    const float cm2 = fmaf(tc, cm1, -cm0);
-    const float sm2 = fmaf(tc, sm1, -sm0);
     float stp0 = 1.0f; (void)stp0;
-    const float stp1 = stp0 * st;
-    const float stp2 = stp1 * st;
     {
         float R = 0x1.20dd76p-2f;
         Y[0] = R;
@@ -963,6 +959,7 @@ template <> __device__ __forceinline__ void sh_basis<2>(
         R = fmaf(R, u, -0x1.42f602p-2f);
         Y[3] = R;
     }
+    const float stp1 = stp0 * st;
     {
         float R = -0x1.17b142p+0f;
         R = R * ct;
@@ -970,6 +967,9 @@ template <> __device__ __forceinline__ void sh_basis<2>(
         Y[4] = P * cm1;
         Y[2] = P * sm1;
     }
+    const float cm2 = fmaf(tc, cm1, -cm0);
+    const float sm2 = fmaf(tc, sm1, -sm0);
+    const float stp2 = stp1 * st;
     {
         float R = 0x1.17b142p-1f;
         const float P = R * stp2;
@@ -986,17 +986,7 @@ template <> __device__ __forceinline__ void sh_basis<4>(
     (void)u;
     const float cm0 = 1.0f, sm0 = 0.0f; (void)cm0; (void)sm0;
     float cm1 = cp, sm1 = sp;
-    const float cm2 = fmaf(tc, cm1, -cm0);
-    const float sm2 = fmaf(tc, sm1, -sm0);
-    const float cm3 = fmaf(tc, cm2, -cm1);
-    const float sm3 = fmaf(tc, sm2, -sm1);
-    const float cm4 = fmaf(tc, cm3, -cm2);
-    const float sm4 = fmaf(tc, sm3, -sm2);
     float stp0 = 1.0f; (void)stp0;
-    const float stp1 = stp0 * st;
-    const float stp2 = stp1 * st;
-    const float stp3 = stp2 * st;
-    const float stp4 = stp3 * st;
     {
         float R = 0x1.20dd76p-2f;
         Y[0] = R;
@@ -1012,6 +1002,7 @@ template <> __device__ __forceinline__ void sh_basis<4>(
         R = fmaf(R, u, 0x1.44f924p-2f);
         Y[10] = R;
     }
+    const float stp1 = stp0 * st;
     {
         float R = -0x1.17b142p+0f;
         R = R * ct;
@@ -1027,6 +1018,9 @@ template <> __device__ __forceinline__ void sh_basis<4>(
         Y[11] = P * cm1;
         Y[9] = P * sm1;
     }
+    const float cm2 = fmaf(tc, cm1, -cm0);
+    const float sm2 = fmaf(tc, sm1, -sm0);
+    const float stp2 = stp1 * st;
     {
         float R = 0x1.17b142p-1f;
         const float P = R * stp2;
@@ -1040,6 +1034,9 @@ template <> __device__ __forceinline__ void sh_basis<4>(
         Y[12] = P * cm2;
         Y[8] = P * sm2;
     }
+    const float cm3 = fmaf(tc, cm2, -cm1);
+    const float sm3 = fmaf(tc, sm2, -sm1);
+    const float stp3 = stp2 * st;
     {
         float R = -0x1.c5274ap+0f;
         R = R * ct;
@@ -1047,6 +1044,9 @@ template <> __device__ __forceinline__ void sh_basis<4>(
         Y[13] = P * cm3;
         Y[7] = P * sm3;
     }
+    const float cm4 = fmaf(tc, cm3, -cm2);
+    const float sm4 = fmaf(tc, sm3, -sm2);
+    const float stp4 = stp3 * st;
     {
         float R = 0x1.406d8ap-1f;
         const float P = R * stp4;
@@ -1063,23 +1063,7 @@ template <> __device__ __forceinline__ void sh_basis<6>(
     (void)u;
     const float cm0 = 1.0f, sm0 = 0.0f; (void)cm0; (void)sm0;
     float cm1 = cp, sm1 = sp;
-    const float cm2 = fmaf(tc, cm1, -cm0);
-    const float sm2 = fmaf(tc, sm1, -sm0);
-    const float cm3 = fmaf(tc, cm2, -cm1);
-    const float sm3 = fmaf(tc, sm2, -sm1);
-    const float cm4 = fmaf(tc, cm3, -cm2);
-    const float sm4 = fmaf(tc, sm3, -sm2);
-    const float cm5 = fmaf(tc, cm4, -cm3);
-    const float sm5 = fmaf(tc, sm4, -sm3);
-    const float cm6 = fmaf(tc, cm5, -cm4);
-    const float sm6 = fmaf(tc, sm5, -sm4);
     float stp0 = 1.0f; (void)stp0;
-    const float stp1 = stp0 * st;
-    const float stp2 = stp1 * st;
-    const float stp3 = stp2 * st;
-    const float stp4 = stp3 * st;
-    const float stp5 = stp4 * st;
-    const float stp6 = stp5 * st;
     {
         float R = 0x1.20dd76p-2f;
         Y[0] = R;
@@ -1102,6 +1086,7 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         R = fmaf(R, u, -0x1.45796cp-2f);
         Y[21] = R;
     }
+    const float stp1 = stp0 * st;
     {
         float R = -0x1.17b142p+0f;
         R = R * ct;
@@ -1126,6 +1111,9 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         Y[22] = P * cm1;
         Y[20] = P * sm1;
     }
+    const float cm2 = fmaf(tc, cm1, -cm0);
+    const float sm2 = fmaf(tc, sm1, -sm0);
+    const float stp2 = stp1 * st;
     {
         float R = 0x1.17b142p-1f;
         const float P = R * stp2;
@@ -1147,6 +1135,9 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         Y[23] = P * cm2;
         Y[19] = P * sm2;
     }
+    const float cm3 = fmaf(tc, cm2, -cm1);
+    const float sm3 = fmaf(tc, sm2, -sm1);
+    const float stp3 = stp2 * st;
     {
         float R = -0x1.c5274ap+0f;
         R = R * ct;
@@ -1162,6 +1153,9 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         Y[24] = P * cm3;
         Y[18] = P * sm3;
     }
+    const float cm4 = fmaf(tc, cm3, -cm2);
+    const float sm4 = fmaf(tc, sm3, -sm2);
+    const float stp4 = stp3 * st;
     {
         float R = 0x1.406d8ap-1f;
         const float P = R * stp4;
@@ -1175,6 +1169,9 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         Y[25] = P * cm4;
         Y[17] = P * sm4;
     }
+    const float cm5 = fmaf(tc, cm4, -cm3);
+    const float sm5 = fmaf(tc, sm4, -sm3);
+    const float stp5 = stp4 * st;
     {
         float R = -0x1.2eed60p+1f;
         R = R * ct;
@@ -1182,6 +1179,9 @@ template <> __device__ __forceinline__ void sh_basis<6>(
         Y[26] = P * cm5;
         Y[16] = P * sm5;
     }
+    const float cm6 = fmaf(tc, cm5, -cm4);
+    const float sm6 = fmaf(tc, sm5, -sm4);
+    const float stp6 = stp5 * st;
     {
         float R = 0x1.5dca4ep-1f;
         const float P = R * stp6;
@@ -1198,29 +1198,7 @@ template <> __device__ __forceinline__ void sh_basis<8>(
     (void)u;
     const float cm0 = 1.0f, sm0 = 0.0f; (void)cm0; (void)sm0;
     float cm1 = cp, sm1 = sp;
-    const float cm2 = fmaf(tc, cm1, -cm0);
-    const float sm2 = fmaf(tc, sm1, -sm0);
-    const float cm3 = fmaf(tc, cm2, -cm1);
-    const float sm3 = fmaf(tc, sm2, -sm1);
-    const float cm4 = fmaf(tc, cm3, -cm2);
-    const float sm4 = fmaf(tc, sm3, -sm2);
-    const float cm5 = fmaf(tc, cm4, -cm3);
-    const float sm5 = fmaf(tc, sm4, -sm3);
-    const float cm6 = fmaf(tc, cm5, -cm4);
-    const float sm6 = fmaf(tc, sm5, -sm4);
-    const float cm7 = fmaf(tc, cm6, -cm5);
-    const float sm7 = fmaf(tc, sm6, -sm5);
-    const float cm8 = fmaf(tc, cm7, -cm6);
-    const float sm8 = fmaf(tc, sm7, -sm6);
     float stp0 = 1.0f; (void)stp0;
-    const float stp1 = stp0 * st;
-    const float stp2 = stp1 * st;
-    const float stp3 = stp2 * st;
-    const float stp4 = stp3 * st;
-    const float stp5 = stp4 * st;
-    const float stp6 = stp5 * st;
-    const float stp7 = stp6 * st;
-    const float stp8 = stp7 * st;
     {
         float R = 0x1.20dd76p-2f;
         Y[0] = R;
@@ -1251,6 +1229,7 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         R = fmaf(R, u, 0x1.45ab7cp-2f);
         Y[36] = R;
     }
+    const float stp1 = stp0 * st;
     {
         float R = -0x1.17b142p+0f;
         R = R * ct;
@@ -1285,6 +1264,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[37] = P * cm1;
         Y[35] = P * sm1;
     }
+    const float cm2 = fmaf(tc, cm1, -cm0);
+    const float sm2 = fmaf(tc, sm1, -sm0);
+    const float stp2 = stp1 * st;
     {
         float R = 0x1.17b142p-1f;
         const float P = R * stp2;
@@ -1315,6 +1297,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[38] = P * cm2;
         Y[34] = P * sm2;
     }
+    const float cm3 = fmaf(tc, cm2, -cm1);
+    const float sm3 = fmaf(tc, sm2, -sm1);
+    const float stp3 = stp2 * st;
     {
         float R = -0x1.c5274ap+0f;
         R = R * ct;
@@ -1339,6 +1324,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[39] = P * cm3;
         Y[33] = P * sm3;
     }
+    const float cm4 = fmaf(tc, cm3, -cm2);
+    const float sm4 = fmaf(tc, sm3, -sm2);
+    const float stp4 = stp3 * st;
     {
         float R = 0x1.406d8ap-1f;
         const float P = R * stp4;
@@ -1360,6 +1348,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[40] = P * cm4;
         Y[32] = P * sm4;
     }
+    const float cm5 = fmaf(tc, cm4, -cm3);
+    const float sm5 = fmaf(tc, sm4, -sm3);
+    const float stp5 = stp4 * st;
     {
         float R = -0x1.2eed60p+1f;
         R = R * ct;
@@ -1375,6 +1366,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[41] = P * cm5;
         Y[31] = P * sm5;
     }
+    const float cm6 = fmaf(tc, cm5, -cm4);
+    const float sm6 = fmaf(tc, sm5, -sm4);
+    const float stp6 = stp5 * st;
     {
         float R = 0x1.5dca4ep-1f;
         const float P = R * stp6;
@@ -1388,6 +1382,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[42] = P * cm6;
         Y[30] = P * sm6;
     }
+    const float cm7 = fmaf(tc, cm6, -cm5);
+    const float sm7 = fmaf(tc, sm6, -sm5);
+    const float stp7 = stp6 * st;
     {
         float R = -0x1.7535e0p+1f;
         R = R * ct;
@@ -1395,6 +1392,9 @@ template <> __device__ __forceinline__ void sh_basis<8>(
         Y[43] = P * cm7;
         Y[29] = P * sm7;
     }
+    const float cm8 = fmaf(tc, cm7, -cm6);
+    const float sm8 = fmaf(tc, sm7, -sm6);
+    const float stp8 = stp7 * st;
     {
         float R = 0x1.7535e0p-1f;
         const float P = R * stp8;

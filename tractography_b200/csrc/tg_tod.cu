@@ -29,20 +29,35 @@ namespace tg {
 namespace {
 
 constexpr int kTodCoefficients = 45;
+// A thread's 45 sums, four to a shared-memory access: the step is bound by
+// instruction issue, and one float at a time took 135 load, add and store
+// instructions of its 820 (40k Transport tracks of 60 mm in 96x96x60: 122 ms a
+// call, 104 ms with quads, the frame shared with the update and a stop test
+// without a root).
+constexpr int kTodQuads = (kTodCoefficients + 3) / 4;
 constexpr int kTodThreads = 128;
 
-__device__ __forceinline__ void tod_flush(float* __restrict__ out, const float* acc, int tid, int ix, int iy, int iz,
+__device__ __forceinline__ void tod_flush(float* __restrict__ out, const float4* acc, int tid, int ix, int iy, int iz,
                                           const TodParams& q)
 {
-    const size_t base = (((size_t)ix * q.ny + iy) * q.nz + iz) * kTodCoefficients;
-#pragma unroll 5
-    for (int k = 0; k < kTodCoefficients; ++k) atomicAdd(out + base + k, acc[k * kTodThreads + tid]);
+    float* dst = out + (((size_t)ix * q.ny + iy) * q.nz + iz) * kTodCoefficients;
+#pragma unroll 1
+    for (int k = 0; k < kTodQuads; ++k) {
+        const float4 v = acc[k * kTodThreads + tid];
+        atomicAdd(dst + 4 * k, v.x);
+        if (4 * k + 1 < kTodCoefficients) {
+            atomicAdd(dst + 4 * k + 1, v.y);
+            atomicAdd(dst + 4 * k + 2, v.z);
+            atomicAdd(dst + 4 * k + 3, v.w);
+        }
+    }
 }
+static_assert(kTodCoefficients % 4 == 1, "the last quad holds one coefficient");
 
 template <int MODEL, int LMAX, int ALGO, int DOM>
 __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
 {
-    __shared__ float acc[kTodCoefficients * kTodThreads];
+    __shared__ float4 acc[kTodQuads * kTodThreads];
     constexpr int CPAD = ModelShape<MODEL, LMAX>::CPAD;
     const int tid = threadIdx.x;
     const TrackParams& p = q.t;
@@ -79,6 +94,7 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
         bool go = live && step < q.n_steps && locate<MODEL, LMAX, CPAD, DOM>(p, s, c);
         __syncwarp();          // join locate()'s exits before the update (track_step)
         if (go) {
+            const Frame f = frame_of(s.ox, s.oy, s.oz);
             // output voxel nearest the point, floor(A^-1 p + 0.5) (tracking.py:294-300)
             const float vx = floorf(dot4(q.out_row0, s.px, s.py, s.pz, 1.0f) + 0.5f);
             const float vy = floorf(dot4(q.out_row1, s.px, s.py, s.pz, 1.0f) + 0.5f);
@@ -86,29 +102,35 @@ __global__ void __launch_bounds__(kTodThreads) tod_kernel(const TodParams q)
             if (vx >= 0.0f && vx < (float)q.nx && vy >= 0.0f && vy < (float)q.ny && vz >= 0.0f &&
                 vz < (float)q.nz) {
                 const int ix = (int)vx, iy = (int)vy, iz = (int)vz;
-                float Y[kTodCoefficients];
-                const Frame f = frame_of(s.ox, s.oy, s.oz);
-                sh_basis<8>(f.ct, f.st, f.cp, f.sp, Y);
-                if (ix == prev_x && iy == prev_y && iz == prev_z) {
-#pragma unroll
-                    for (int k = 0; k < kTodCoefficients; ++k) acc[k * kTodThreads + tid] += Y[k];
-                } else {
+                if (ix != prev_x || iy != prev_y || iz != prev_z) {
+                    // a new voxel starts from zero (0 + Y = Y), so that the sum
+                    // below is one piece of code for every lane
                     if (prev_x >= 0) tod_flush(q.coefficients, acc, tid, prev_x, prev_y, prev_z, q);
 #pragma unroll
-                    for (int k = 0; k < kTodCoefficients; ++k) acc[k * kTodThreads + tid] = Y[k];
+                    for (int k = 0; k < kTodQuads; ++k) acc[k * kTodThreads + tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     prev_x = ix;
                     prev_y = iy;
                     prev_z = iz;
+                }
+                float Y[4 * kTodQuads];
+                sh_basis<8>(f.ct, f.st, f.cp, f.sp, Y);
+                Y[45] = Y[46] = Y[47] = 0.0f;
+#pragma unroll
+                for (int k = 0; k < kTodQuads; ++k) {
+                    float4 v = acc[k * kTodThreads + tid];
+                    v.x += Y[4 * k];
+                    v.y += Y[4 * k + 1];
+                    v.z += Y[4 * k + 2];
+                    v.w += Y[4 * k + 3];
+                    acc[k * kTodThreads + tid] = v;
                 }
             } else if (prev_x >= 0) {
                 tod_flush(q.coefficients, acc, tid, prev_x, prev_y, prev_z, q);
                 prev_x = prev_y = prev_z = -1;
             }
-            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
+            update_orientation<MODEL, LMAX, ALGO>(p.algo, c, f, s.ox, s.oy, s.oz, s.rng, s.steps);
             s.steps += 1u;
-            // tracking.py:343: stop on a non-finite or degenerate orientation
-            const float len = sqrtf(s.ox * s.ox + s.oy * s.oy + s.oz * s.oz);
-            if (!(isfinite(s.ox) && isfinite(s.oy) && isfinite(s.oz)) || len < 0.5f) {
+            if (degenerate(s.ox, s.oy, s.oz)) {
                 go = false;
             } else {
                 const float h = p.algo.step_size;
