@@ -76,6 +76,14 @@ __host__ __device__ __forceinline__ void mesh_ray(int r, float& x, float& y, flo
 
 // One segment start + t * d, t in [0, 1], with the per-axis reciprocals
 // bvh.cl:32 recomputes per node (same IEEE division, same value).
+__device__ __forceinline__ float rcp_signed(float x)
+{
+    // tgm_rcp's Newton step for either sign; anything outside its range
+    // (zero and infinity among it) takes the division
+    if (fabsf(x) >= 0x1p-125f && fabsf(x) < 0x1p125f) return copysignf(tgm_rcp(fabsf(x)), x);
+    return 1.0f / x;
+}
+
 struct Segment {
     float sx, sy, sz;
     float dx, dy, dz;
@@ -91,9 +99,9 @@ __device__ __forceinline__ Segment make_segment(float sx, float sy, float sz, fl
     g.px = fabsf(g.dx) < 1e-12f;
     g.py = fabsf(g.dy) < 1e-12f;
     g.pz = fabsf(g.dz) < 1e-12f;
-    g.ix = 1.0f / g.dx;
-    g.iy = 1.0f / g.dy;
-    g.iz = 1.0f / g.dz;
+    g.ix = rcp_signed(g.dx);
+    g.iy = rcp_signed(g.dy);
+    g.iz = rcp_signed(g.dz);
     return g;
 }
 
@@ -116,12 +124,26 @@ __device__ __forceinline__ bool slab(bool parallel, float s, float inv, float lo
     return !(t0 > t1);
 }
 
+// Without a parallel axis the three slabs are evaluated without branches, which
+// split a warp three ways here: t0 only grows and t1 only shrinks, so one
+// comparison at the end says what the comparison after each axis would, and
+// min / max differ from the compare-and-select forms above in nothing but the
+// sign of a zero, which no comparison sees, and NaN: one among the slabs leaves
+// t0 and t1 as they are in both, and a NaN max_t (a hit's t after overflow) stays.
 __device__ __forceinline__ bool box_hit(const Segment& g, float4 lo, float4 hi, float max_t)
 {
     float t0 = 0.0f, t1 = max_t;
-    if (!slab(g.px, g.sx, g.ix, lo.x, hi.x, t0, t1)) return false;
-    if (!slab(g.py, g.sy, g.iy, lo.y, hi.y, t0, t1)) return false;
-    return slab(g.pz, g.sz, g.iz, lo.z, hi.z, t0, t1);
+    if (g.px || g.py || g.pz) {
+        if (!slab(g.px, g.sx, g.ix, lo.x, hi.x, t0, t1)) return false;
+        if (!slab(g.py, g.sy, g.iy, lo.y, hi.y, t0, t1)) return false;
+        return slab(g.pz, g.sz, g.iz, lo.z, hi.z, t0, t1);
+    }
+    const float ax = (lo.x - g.sx) * g.ix, bx = (hi.x - g.sx) * g.ix;
+    const float ay = (lo.y - g.sy) * g.iy, by = (hi.y - g.sy) * g.iy;
+    const float az = (lo.z - g.sz) * g.iz, bz = (hi.z - g.sz) * g.iz;
+    t0 = fmaxf(fmaxf(t0, fminf(ax, bx)), fmaxf(fminf(ay, by), fminf(az, bz)));
+    t1 = cl_min(t1, fminf(fmaxf(ax, bx), fminf(fmaxf(ay, by), fmaxf(az, bz))));
+    return !(t0 > t1);
 }
 
 // bvh.cl:47-80 (Moller-Trumbore, the reference's tolerances).
@@ -137,7 +159,7 @@ __device__ __forceinline__ bool triangle_hit(const Segment& g, const float4* tri
     const float pz = g.dx * e2.y - g.dy * e2.x;
     const float det = e1.x * px + e1.y * py + e1.z * pz;
     if (fabsf(det) < 1e-10f) return false;
-    const float inv_det = 1.0f / det;
+    const float inv_det = rcp_signed(det);
     const float ox = g.sx - a.x, oy = g.sy - a.y, oz = g.sz - a.z;
     const float u = (ox * px + oy * py + oz * pz) * inv_det;
     if (u < -1e-6f || u > 1.0f + 1e-6f) return false;
@@ -155,8 +177,26 @@ __device__ __forceinline__ bool triangle_hit(const Segment& g, const float4* tri
     return true;
 }
 
-// MODE 0: closest hit (bvh.cl:83-131); 1: any hit, stop at the first;
-// 2: count every hit with max_t fixed at 1.
+// The next leaf in walk order from node i on whose box the segment hits
+// within max_t: its code (triangles), or -1 at the end of the tree; i moves past
+// it.  A loop of its own, so that a warp's lanes meet with a leaf each before any
+// of them tests triangles: in one loop over nodes, nearly every iteration of a
+// warp ran the triangle tests for the few lanes that stood at a leaf.
+__device__ __forceinline__ int next_leaf(const MeshDev& m, const Segment& g, float max_t, uint32_t& i)
+{
+    while (i < m.n_nodes) {
+        const float4 lo = __ldg(m.nodes + 2 * (size_t)i);
+        const float4 hi = __ldg(m.nodes + 2 * (size_t)i + 1);
+        const int code = __float_as_int(hi.w);
+        const bool hit = box_hit(g, lo, hi, max_t);
+        // down, or past the subtree (a leaf's too)
+        i = hit && code < 0 ? i + 1u : __float_as_uint(lo.w);
+        if (hit && code >= 0) return code;
+    }
+    return -1;
+}
+
+// MODE 0: closest hit (bvh.cl:83-131); 1: any hit, stop at the first.
 template <int MODE>
 __device__ __forceinline__ uint32_t mesh_walk(const MeshDev& m, const Segment& g, float& t, uint32_t& tri,
                                               float& u, float& v)
@@ -165,60 +205,97 @@ __device__ __forceinline__ uint32_t mesh_walk(const MeshDev& m, const Segment& g
     tri = 0u;
     uint32_t hits = 0u;
     uint32_t i = 0u;
-    while (i < m.n_nodes) {
-        const float4 lo = __ldg(m.nodes + 2 * (size_t)i);
-        const float4 hi = __ldg(m.nodes + 2 * (size_t)i + 1);
-        const uint32_t skip = __float_as_uint(lo.w);
-        if (!box_hit(g, lo, hi, MODE == 2 ? 1.0f : t)) {
-            i = skip;
-            continue;
-        }
-        const int code = __float_as_int(hi.w);
-        if (code < 0) {
-            i = i + 1u;
-            continue;
-        }
+    while (true) {
+        const int code = next_leaf(m, g, t, i);
+        if (code < 0) break;
         const uint32_t first = (uint32_t)code >> 3;
         const uint32_t count = (uint32_t)code & 7u;
         for (uint32_t k = 0; k < count; ++k) {
             const float4* tp = m.tris + 3 * (size_t)(first + k);
             float tt, uu, vv;
-            if (triangle_hit(g, tp, MODE == 2 ? 1.0f : t, tt, uu, vv)) {
+            if (triangle_hit(g, tp, t, tt, uu, vv)) {
                 hits += 1u;
                 if (MODE == 0) {
                     t = tt;
                     u = uu;
                     v = vv;
                     tri = __float_as_uint(__ldg(tp).w);
-                } else if (MODE == 1) {
+                } else {
                     return 1u;
                 }
             }
         }
-        i = skip;
     }
     return hits;
 }
 
-// Inside test: majority over three rays of the parity of crossings; points
-// outside the root bounds are outside.
+// Inside test: majority over three rays of the parity of crossings (the third
+// ray only where the first two disagree); points outside the root bounds are
+// outside.  The test as a state machine, one leaf's triangles per advance(), so
+// that a kernel's lanes take their next ray or point as soon as they are done
+// with one instead of waiting for the longest ray of their warp.
+struct InsideTest {
+    float x, y, z;
+    Segment g;
+    uint32_t node;
+    uint32_t crossings;
+    int ray, odd;
+
+    __device__ __forceinline__ void aim(const MeshDev& m)
+    {
+        const float4 lo = __ldg(m.nodes);
+        const float4 hi = __ldg(m.nodes + 1);
+        const float reach = (((hi.x - lo.x) + (hi.y - lo.y)) + (hi.z - lo.z)) + 1.0f;
+        float rx, ry, rz;
+        mesh_ray(ray, rx, ry, rz);
+        g = make_segment(x, y, z, x + reach * rx, y + reach * ry, z + reach * rz);
+        node = 0u;
+        crossings = 0u;
+    }
+
+    // false: the point lies outside the root bounds.
+    __device__ __forceinline__ bool start(const MeshDev& m, float px, float py, float pz)
+    {
+        const float4 lo = __ldg(m.nodes);
+        const float4 hi = __ldg(m.nodes + 1);
+        if (!(px >= lo.x && px <= hi.x && py >= lo.y && py <= hi.y && pz >= lo.z && pz <= hi.z)) return false;
+        x = px;
+        y = py;
+        z = pz;
+        ray = 0;
+        odd = 0;
+        aim(m);
+        return true;
+    }
+
+    // One more leaf; true when the answer (odd >= 2) stands.
+    __device__ __forceinline__ bool advance(const MeshDev& m)
+    {
+        const int code = next_leaf(m, g, 1.0f, node);
+        if (code >= 0) {
+            const uint32_t first = (uint32_t)code >> 3;
+            const uint32_t count = (uint32_t)code & 7u;
+            for (uint32_t k = 0; k < count; ++k) {
+                float t, u, v;
+                if (triangle_hit(g, m.tris + 3 * (size_t)(first + k), 1.0f, t, u, v)) crossings += 1u;
+            }
+            return false;
+        }
+        odd += (int)(crossings & 1u);
+        ray += 1;
+        if (ray == 3 || (ray == 2 && odd != 1)) return true;
+        aim(m);
+        return false;
+    }
+};
+
 __device__ __forceinline__ bool mesh_contains(const MeshDev& m, float x, float y, float z)
 {
-    const float4 lo = __ldg(m.nodes);
-    const float4 hi = __ldg(m.nodes + 1);
-    if (!(x >= lo.x && x <= hi.x && y >= lo.y && y <= hi.y && z >= lo.z && z <= hi.z)) return false;
-    const float reach = (((hi.x - lo.x) + (hi.y - lo.y)) + (hi.z - lo.z)) + 1.0f;
-    int odd = 0;
-#pragma unroll 1
-    for (int r = 0; r < 3; ++r) {
-        float rx, ry, rz;
-        mesh_ray(r, rx, ry, rz);
-        const Segment g = make_segment(x, y, z, x + reach * rx, y + reach * ry, z + reach * rz);
-        float t, u, v;
-        uint32_t tri;
-        odd += (int)(mesh_walk<2>(m, g, t, tri, u, v) & 1u);
+    InsideTest q;
+    if (!q.start(m, x, y, z)) return false;
+    while (!q.advance(m)) {
     }
-    return odd >= 2;
+    return q.odd >= 2;
 }
 
 // Any hit among the leaves of one cell's list (count, then leaf node

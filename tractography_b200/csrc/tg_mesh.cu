@@ -419,10 +419,27 @@ __global__ void __launch_bounds__(128) mesh_segment_hits_kernel(MeshDev m, const
 __global__ void __launch_bounds__(128) mesh_contains_kernel(MeshDev m, const float4* __restrict__ points,
                                                             uint32_t n, uint32_t stride, uint8_t* __restrict__ out)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = points[(size_t)i * stride];
-    out[i] = mesh_contains(m, p.x, p.y, p.z) ? 1 : 0;
+    // Points i, i + threads, ...: a lane goes on to its next point when the
+    // answer for one stands.
+    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    InsideTest q;
+    bool busy = false;
+    while (true) {
+        while (!busy && i < n) {
+            const float4 p = points[(size_t)i * stride];
+            busy = q.start(m, p.x, p.y, p.z);
+            if (!busy) {
+                out[i] = 0;
+                i += (uint64_t)gridDim.x * blockDim.x;
+            }
+        }
+        if (!busy) break;
+        if (q.advance(m)) {
+            out[i] = q.odd >= 2 ? 1 : 0;
+            i += (uint64_t)gridDim.x * blockDim.x;
+            busy = false;
+        }
+    }
 }
 
 __global__ void __launch_bounds__(128) mesh_segments_blocked_kernel(MeshDev m, const float4* __restrict__ starts,
@@ -455,7 +472,13 @@ cudaError_t launch_mesh_contains(const MeshDev& m, const float4* points, uint32_
                                  cudaStream_t stream, uint32_t stride)
 {
     if (n == 0) return cudaSuccess;
-    mesh_contains_kernel<<<(n + 127) / 128, 128, 0, stream>>>(m, points, n, stride, out);
+    int dev = 0, sms = 148, per_sm = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mesh_contains_kernel, 128, 0) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const uint32_t want = (n - 1) / 128 + 1, full = (uint32_t)(sms * per_sm);
+    mesh_contains_kernel<<<want < full ? want : full, 128, 0, stream>>>(m, points, n, stride, out);
     return cudaGetLastError();
 }
 
