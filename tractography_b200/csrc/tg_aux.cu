@@ -9,6 +9,7 @@
  *   update_orientation_kernel algorithm.py:738-759 (tg.algorithm.update_orientation)
  *   rng_stream_kernel        core.cl:218-238 (randus / randis test streams)
  */
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
 #include "tg_internal.h"
@@ -33,92 +34,241 @@ __device__ __forceinline__ float3 fibonacci(uint32_t n, uint32_t n_points)
     return make_float3(radius * c, radius * s, z);
 }
 
-// Table of the 1000 directions (float4, w = 0) and, for SH, the basis
-// values Y_i at each direction, rows of `cpad` floats.
-template <int LMAX>
-__global__ void fod_table_kernel(float4* dirs, float* Y, int cpad, int is_sh)
+// The 1000 directions (w = 0) and the basis values Y_i at each, rows of CPAD
+// floats per band limit.  In module memory: allocating them on each call took
+// longer than the kernels (the stream-ordered pool gives its memory back at
+// every synchronisation).  Every call writes its band's table again, always with
+// the same bits, so calls on several streams do not disturb one another.
+__device__ float4 g_fod_dirs[kDirections];
+
+__host__ __device__ constexpr int fod_row(int lmax) { return (n_coef_full(lmax) + 3) / 4; }     // float4s
+__host__ __device__ constexpr int fod_table_at(int lmax)
+{
+    return lmax == 0 ? 0 : fod_table_at(lmax - 2) + kDirections * fod_row(lmax - 2);
+}
+__device__ float4 g_fod_tables[fod_table_at(8) + kDirections * fod_row(8)];
+
+template <int MODEL, int LMAX>
+__global__ void fod_table_kernel()
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kDirections) return;
     const float3 d = fibonacci((uint32_t)i, kDirections);
-    dirs[i] = make_float4(d.x, d.y, d.z, 0.0f);
-    if (is_sh) {
-        float row[n_coef_full(LMAX)];
+    g_fod_dirs[i] = make_float4(d.x, d.y, d.z, 0.0f);
+    if constexpr (MODEL == kModelSH) {
+        constexpr int N = n_coef_full(LMAX), ROW = fod_row(LMAX);
+        float row[4 * ROW];
         const Frame f = frame_of(d.x, d.y, d.z);
         sh_basis<LMAX>(f.ct, f.st, f.cp, f.sp, row);
-        for (int j = 0; j < cpad; ++j) Y[(size_t)i * cpad + j] = j < n_coef_full(LMAX) ? row[j] : 0.0f;
+#pragma unroll
+        for (int j = N; j < 4 * ROW; ++j) row[j] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < ROW; ++k)
+            g_fod_tables[fod_table_at(LMAX) + i * ROW + k] =
+                make_float4(row[4 * k], row[4 * k + 1], row[4 * k + 2], row[4 * k + 3]);
     }
 }
 
-template <int MODEL, int CPAD>
-__device__ __forceinline__ float fod_value(const float (&c)[CPAD], uint32_t C, const float4* dirs,
-                                           const float* Y, int i)
+// The model's values of S seeds at one direction, floored at 0; row: the
+// direction's basis values, or the direction itself for tensors.
+template <int MODEL, int LMAX, int CPAD, int S>
+__device__ __forceinline__ void fod_values(const float (&c)[S][CPAD], const float4* row, float (&value)[S])
 {
     if constexpr (MODEL == kModelDTI) {
-        const float4 d = __ldg(dirs + i);
+        const float4 d = row[0];
         const Frame f = frame_of(d.x, d.y, d.z);
-        return dti_model(c, d.x, d.y, d.z, f).value;
+#pragma unroll
+        for (int s = 0; s < S; ++s) value[s] = dti_model(c[s], d.x, d.y, d.z, f).value;
     } else {
-        const float4* row = reinterpret_cast<const float4*>(Y + (size_t)i * CPAD);
-        float raw = 0.0f;
+        float raw[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) raw[s] = 0.0f;
 #pragma unroll
         for (int k = 0; k < CPAD / 4; ++k) {
-            const float4 y = __ldg(row + k);
-            if (4 * k + 0 < (int)C) raw = fmaf(c[4 * k + 0], y.x, raw);
-            if (4 * k + 1 < (int)C) raw = fmaf(c[4 * k + 1], y.y, raw);
-            if (4 * k + 2 < (int)C) raw = fmaf(c[4 * k + 2], y.z, raw);
-            if (4 * k + 3 < (int)C) raw = fmaf(c[4 * k + 3], y.w, raw);
+            const float4 y = row[k];
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                raw[s] = fmaf(c[s][4 * k], y.x, raw[s]);
+                if (4 * k + 1 < n_coef_full(LMAX)) raw[s] = fmaf(c[s][4 * k + 1], y.y, raw[s]);
+                if (4 * k + 2 < n_coef_full(LMAX)) raw[s] = fmaf(c[s][4 * k + 2], y.z, raw[s]);
+                if (4 * k + 3 < n_coef_full(LMAX)) raw[s] = fmaf(c[s][4 * k + 3], y.w, raw[s]);
+            }
         }
-        return softmax(raw, kSoftmaxScale);
+        if constexpr (S == 2) {
+            const F2 v = softmax2(f2(raw[0], raw[1]));
+            value[0] = lo(v);
+            value[1] = hi(v);
+        } else {
+#pragma unroll
+            for (int s = 0; s < S; ++s) value[s] = softmax(raw[s]);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) value[s] = cl_max(value[s], 0.0f);
+}
+
+// S seeds per thread.  The cumulative sum over the directions is kept every
+// kCheck of them, so that the search for the first one above the threshold
+// evaluates kCheck directions again instead of all 1000.  The basis goes through
+// shared memory kCheck directions at a time, the next ones copied meanwhile.
+// Bound by what it takes to hand a basis row to a warp (12 16-byte loads, four
+// cycles each, at lmax 8) and by instruction issue (45 multiply-adds and a
+// softplus per direction and seed); two seeds per thread share a row's loads
+// and a softplus's instructions.  1M seeds at lmax 8: 15.6 ms as two passes over
+// a table in global memory, 4.2 ms so; 1000 seeds 1.5 and 0.25 ms.
+constexpr int kCheck = 16;
+constexpr int kChecks = (kDirections + kCheck - 1) / kCheck;
+constexpr int kFodThreads = 128;
+
+template <int MODEL, int LMAX>
+struct FodShape {
+    static constexpr int CPAD = MODEL == kModelDTI ? 8 : ModelShape<kModelSH, LMAX>::CPAD;
+    static constexpr int ROW = MODEL == kModelDTI ? 1 : CPAD / 4;       // float4s per direction
+};
+
+template <int MODEL, int LMAX, int S>
+constexpr size_t fod_shared_bytes()
+{
+    return 2 * kCheck * FodShape<MODEL, LMAX>::ROW * sizeof(float4) + (size_t)kChecks * kFodThreads * S * sizeof(float);
+}
+
+template <int MODEL, int LMAX, int S>
+__global__ void __launch_bounds__(kFodThreads) seeds_from_fod_kernel(
+    const float* __restrict__ fod, uint32_t C, const float4* __restrict__ voxels, uint32_t nnz,
+    const float* __restrict__ affine, const uint2* __restrict__ states, uint32_t n_seeds, float4* __restrict__ seeds)
+{
+    constexpr int CPAD = FodShape<MODEL, LMAX>::CPAD, ROW = FodShape<MODEL, LMAX>::ROW;
+    constexpr int kTile = kCheck * ROW;                    // float4s
+    const float4* const table = MODEL == kModelDTI ? g_fod_dirs : g_fod_tables + fod_table_at(LMAX);
+    extern __shared__ float4 fod_shared[];
+    float4* const tile = fod_shared;
+    float* const check = reinterpret_cast<float*>(fod_shared + 2 * kTile);
+    const uint32_t tid = threadIdx.x;
+    float c[S][CPAD];
+    Mwc state[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const uint32_t gid = (blockIdx.x * S + s) * kFodThreads + tid;
+        const uint32_t seed = gid < n_seeds ? gid : n_seeds - 1;   // past the end: the last one again, not written
+        const uint2 st = states[seed];
+        Mwc r;
+        r.x = st.x;
+        r.c = st.y;
+        uint32_t vi = randi(r, nnz);                      // seeds.cl:89
+        if (vi >= nnz) vi = nnz - 1;
+        const float4 v = voxels[vi];
+        float vx = v.x, vy = v.y, vz = v.z;
+        vx = vx + (randu(r) - 0.5f);                      // seeds.cl:94 (x, y, z order)
+        vy = vy + (randu(r) - 0.5f);
+        vz = vz + (randu(r) - 0.5f);
+        state[s] = r;
+#pragma unroll
+        for (int k = 0; k < CPAD; ++k) c[s][k] = (uint32_t)k < C ? fod[(size_t)vi * C + k] : 0.0f;
+        if (gid < n_seeds) {
+            float4 loc;
+            const float4 r0 = make_float4(affine[0], affine[1], affine[2], affine[3]);
+            const float4 r1 = make_float4(affine[4], affine[5], affine[6], affine[7]);
+            const float4 r2 = make_float4(affine[8], affine[9], affine[10], affine[11]);
+            const float4 r3 = make_float4(affine[12], affine[13], affine[14], affine[15]);
+            loc.x = dot4(r0, vx, vy, vz, v.w);
+            loc.y = dot4(r1, vx, vy, vz, v.w);
+            loc.z = dot4(r2, vx, vy, vz, v.w);
+            loc.w = dot4(r3, vx, vy, vz, v.w);
+            seeds[2 * (size_t)gid] = loc;
+        }
+    }
+
+    auto copy_tile = [&](int b) {                          // directions b kCheck .. of the table
+        for (int q = (int)tid; q < kTile && b * kTile + q < kDirections * ROW; q += kFodThreads)
+            __pipeline_memcpy_async(tile + (b & 1) * kTile + q, table + b * kTile + q, sizeof(float4));
+        __pipeline_commit();
+    };
+    float sum[S], value[S];                               // seeds.cl:29-35
+#pragma unroll
+    for (int s = 0; s < S; ++s) sum[s] = 0.0f;
+    copy_tile(0);
+    for (int b = 0; b < kChecks; ++b) {
+        __pipeline_wait_prior(0);
+        __syncthreads();                                  // tile b is there, tile b - 1 read
+        if (b + 1 < kChecks) copy_tile(b + 1);
+        const float4* rows = tile + (b & 1) * kTile;
+        const int n = min(kCheck, kDirections - b * kCheck);
+#pragma unroll 2
+        for (int i = 0; i < n; ++i) {
+            fod_values<MODEL, LMAX, CPAD, S>(c, rows + i * ROW, value);
+#pragma unroll
+            for (int s = 0; s < S; ++s) sum[s] = sum[s] + value[s];
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) check[(b * S + s) * kFodThreads + tid] = sum[s];
+    }
+
+    float threshold[S], cs[S];                            // seeds.cl:38
+    int from[S], selected[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        threshold[s] = randu(state[s]) * sum[s];
+        // first kept sum above the threshold (they never fall; none is above a NaN)
+        int low = 0, high = kChecks;
+        while (low < high) {
+            const int mid = (low + high) / 2;
+            if (check[(mid * S + s) * kFodThreads + tid] > threshold[s]) high = mid;
+            else low = mid + 1;
+        }
+        from[s] = low;
+        cs[s] = low > 0 && low < kChecks ? check[((low - 1) * S + s) * kFodThreads + tid] : 0.0f;
+        selected[s] = kDirections;
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if (from[s] == kChecks) continue;
+        float one[1][CPAD], v[1];
+#pragma unroll
+        for (int k = 0; k < CPAD; ++k) one[0][k] = c[s][k];
+        const int end = min((from[s] + 1) * kCheck, kDirections);
+        for (int i = from[s] * kCheck; i < end; ++i) {
+            fod_values<MODEL, LMAX, CPAD, 1>(one, table + i * ROW, v);
+            cs[s] = cs[s] + v[0];
+            if (cs[s] > threshold[s]) {
+                selected[s] = i;
+                break;
+            }
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const uint32_t gid = (blockIdx.x * S + s) * kFodThreads + tid;
+        if (gid < n_seeds)
+            seeds[2 * (size_t)gid + 1] = selected[s] < kDirections ? g_fod_dirs[selected[s]] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
     }
 }
 
-template <int MODEL, int CPAD>
-__global__ void __launch_bounds__(128) seeds_from_fod_kernel(const float* __restrict__ fod, uint32_t C,
-                                                             const float4* __restrict__ voxels, uint32_t nnz,
-                                                             const float* __restrict__ affine,
-                                                             const uint2* __restrict__ states, uint32_t n_seeds,
-                                                             const float4* __restrict__ dirs,
-                                                             const float* __restrict__ Y,
-                                                             float4* __restrict__ seeds)
+template <int MODEL, int LMAX, int S>
+cudaError_t run_seeds_from_fod(const float* fod, uint32_t C, const float4* voxels, uint32_t nnz, const float* affine,
+                               const uint2* states, uint32_t n_seeds, float4* seeds, cudaStream_t stream)
 {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= n_seeds) return;
-    const uint2 st = states[gid];
-    Mwc s;
-    s.x = st.x;
-    s.c = st.y;
-    uint32_t vi = randi(s, nnz);                          // seeds.cl:89
-    if (vi >= nnz) vi = nnz - 1;
-    const float4 v = voxels[vi];
-    float vx = v.x, vy = v.y, vz = v.z;
-    vx = vx + (randu(s) - 0.5f);                          // seeds.cl:94 (x, y, z order)
-    vy = vy + (randu(s) - 0.5f);
-    vz = vz + (randu(s) - 0.5f);
-    float c[CPAD];
-#pragma unroll
-    for (int k = 0; k < CPAD; ++k) c[k] = (uint32_t)k < C ? fod[(size_t)vi * C + k] : 0.0f;
+    constexpr size_t bytes = fod_shared_bytes<MODEL, LMAX, S>();
+    cudaError_t e = cudaFuncSetAttribute(seeds_from_fod_kernel<MODEL, LMAX, S>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    fod_table_kernel<MODEL, LMAX><<<(kDirections + 31) / 32, 32, 0, stream>>>();
+    seeds_from_fod_kernel<MODEL, LMAX, S><<<(n_seeds - 1) / (kFodThreads * S) + 1, kFodThreads, bytes, stream>>>(
+        fod, C, voxels, nnz, affine, states, n_seeds, seeds);
+    return cudaGetLastError();
+}
 
-    float sum = 0.0f;                                     // seeds.cl:29-35
-    for (int i = 0; i < kDirections; ++i) sum = sum + cl_max(fod_value<MODEL, CPAD>(c, C, dirs, Y, i), 0.0f);
-    const float threshold = randu(s) * sum;               // seeds.cl:38
-    float cs = 0.0f;
-    int selected = kDirections;
-    for (int i = 0; i < kDirections; ++i) {
-        cs = cs + cl_max(fod_value<MODEL, CPAD>(c, C, dirs, Y, i), 0.0f);
-        if (selected == kDirections && cs > threshold) selected = i;
+// Two seeds per thread where one per thread would be more than two warps per
+// scheduler: fewer loads and instructions per seed, but half as many warps to
+// hide their latency.  lmax 8, one and two seeds per thread: 30k seeds 0.281 and
+// 0.334 ms, 100k 0.627 and 0.522 ms, 1M 4.46 and 4.25 ms.  A tensor's row is one
+// load, so two seeds save nothing there (1M: 0.68 and 0.75 ms).
+template <int MODEL, int LMAX, typename... Args>
+cudaError_t seeds_from_fod(uint32_t n_seeds, int sms, Args... args)
+{
+    if constexpr (MODEL == kModelSH) {
+        if (n_seeds > (uint32_t)sms * kFodThreads * 2) return run_seeds_from_fod<MODEL, LMAX, 2>(args...);
     }
-    float4 loc;
-    const float4 r0 = make_float4(affine[0], affine[1], affine[2], affine[3]);
-    const float4 r1 = make_float4(affine[4], affine[5], affine[6], affine[7]);
-    const float4 r2 = make_float4(affine[8], affine[9], affine[10], affine[11]);
-    const float4 r3 = make_float4(affine[12], affine[13], affine[14], affine[15]);
-    loc.x = dot4(r0, vx, vy, vz, v.w);
-    loc.y = dot4(r1, vx, vy, vz, v.w);
-    loc.z = dot4(r2, vx, vy, vz, v.w);
-    loc.w = dot4(r3, vx, vy, vz, v.w);
-    seeds[2 * (size_t)gid] = loc;
-    seeds[2 * (size_t)gid + 1] = selected < kDirections ? dirs[selected] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+    return run_seeds_from_fod<MODEL, LMAX, 1>(args...);
 }
 
 cudaError_t launch_seeds_from_fod(int model, uint32_t C, const float* fod, const float4* voxels, uint32_t nnz,
@@ -126,44 +276,19 @@ cudaError_t launch_seeds_from_fod(int model, uint32_t C, const float* fod, const
                                   cudaStream_t stream)
 {
     if (n_seeds == 0) return cudaSuccess;
-    const int lmax = lmax_for(C);
-    const int cpad = model == kModelDTI ? 8 : (n_coef_full(lmax) + 3) / 4 * 4;
-    float4* dirs = nullptr;
-    float* Y = nullptr;
-    cudaError_t e = cudaMallocAsync(&dirs, kDirections * sizeof(float4), stream);
-    if (e != cudaSuccess) return e;
-    e = cudaMallocAsync(&Y, (size_t)kDirections * cpad * sizeof(float), stream);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(dirs, stream);
-        return e;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#define TG_FOD(M, L) seeds_from_fod<M, L>(n_seeds, sms, fod, C, voxels, nnz, affine, states, n_seeds, seeds, stream)
+    if (model == kModelDTI) return TG_FOD(kModelDTI, 0);
+    switch (lmax_for(C)) {
+    case 0: return TG_FOD(kModelSH, 0);
+    case 2: return TG_FOD(kModelSH, 2);
+    case 4: return TG_FOD(kModelSH, 4);
+    case 6: return TG_FOD(kModelSH, 6);
+    default: return TG_FOD(kModelSH, 8);
     }
-    const int is_sh = model == kModelSH;
-    const int tb = 128, tg_ = (kDirections + tb - 1) / tb;
-    switch (is_sh ? lmax : 0) {
-    case 0: fod_table_kernel<0><<<tg_, tb, 0, stream>>>(dirs, Y, cpad, is_sh); break;
-    case 2: fod_table_kernel<2><<<tg_, tb, 0, stream>>>(dirs, Y, cpad, is_sh); break;
-    case 4: fod_table_kernel<4><<<tg_, tb, 0, stream>>>(dirs, Y, cpad, is_sh); break;
-    case 6: fod_table_kernel<6><<<tg_, tb, 0, stream>>>(dirs, Y, cpad, is_sh); break;
-    default: fod_table_kernel<8><<<tg_, tb, 0, stream>>>(dirs, Y, cpad, is_sh); break;
-    }
-    const int block = 128;
-    const int grid = (int)((n_seeds + block - 1) / block);
-    if (model == kModelDTI) {
-        seeds_from_fod_kernel<kModelDTI, 8><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states,
-                                                                        n_seeds, dirs, Y, seeds);
-    } else {
-        switch (cpad) {
-        case 4: seeds_from_fod_kernel<kModelSH, 4><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states, n_seeds, dirs, Y, seeds); break;
-        case 8: seeds_from_fod_kernel<kModelSH, 8><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states, n_seeds, dirs, Y, seeds); break;
-        case 16: seeds_from_fod_kernel<kModelSH, 16><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states, n_seeds, dirs, Y, seeds); break;
-        case 28: seeds_from_fod_kernel<kModelSH, 28><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states, n_seeds, dirs, Y, seeds); break;
-        default: seeds_from_fod_kernel<kModelSH, 48><<<grid, block, 0, stream>>>(fod, C, voxels, nnz, affine, states, n_seeds, dirs, Y, seeds); break;
-        }
-    }
-    e = cudaGetLastError();
-    cudaFreeAsync(Y, stream);
-    cudaFreeAsync(dirs, stream);
-    return e;
+#undef TG_FOD
 }
 
 // ------------------------------------------------------------ unit hooks

@@ -303,11 +303,91 @@ struct ModelValue {
     float inv;   // 1 / max(value, 1e-6), the drift's divisor (algorithm.py:98, :216)
 };
 
-// core.cl:111-115 (the seeding kernel's model value; tracking uses tgm_softplus)
-__device__ __forceinline__ float softmax(float x, float k)
+// core.cl:111-115, log(1 + e^{kx}) / k below kx = 30, else x: the seeding kernel's
+// model value (tracking uses tgm_softplus).  tgm_expf, tgm_logf and the two
+// divisions in their operations, for the arguments that occur here: 1 + e is
+// in [1, 1 + e^30] (and 1 wherever the exponential is below 2^-24, so its
+// argument may be capped), and both quotients are one Newton step with a fused
+// residual from the reciprocal (Markstein 1990, as in tgm_rcp).  Equal to
+// tgm_logf(1 + tgm_expf(kx)) / k on all 2^32 floats (checked exhaustively on B200)
+// in half its instructions.
+__device__ __forceinline__ float softmax(float x)
 {
-    if (x * k < 30.0f) return tgm_logf(1.0f + tgm_expf(k * x)) / k;
-    return x;
+    const float kx = x * kSoftmaxScale;
+    const float y = fminf(fmaxf(kx, -87.0f), 30.0f);
+    const float shifted = y * TGM_LOG2E + 0x1.8p+23f;
+    const float k = shifted - 0x1.8p+23f;
+    float r = fmaf(-k, TGM_LN2_HI, y);
+    r = fmaf(-k, TGM_LN2_LO, r);
+    float p = 0x1.a01a02p-13f;
+    p = fmaf(p, r, 0x1.6c16c2p-10f);
+    p = fmaf(p, r, 0x1.111112p-7f);
+    p = fmaf(p, r, 0x1.555556p-5f);
+    p = fmaf(p, r, 0x1.555556p-3f);
+    p = fmaf(p, r, 0.5f);
+    p = fmaf(p, r, 1.0f);
+    p = fmaf(p, r, 1.0f);
+    const float w = 1.0f + p * __uint_as_float((__float_as_uint(shifted) << 23) + 0x3f800000u);
+    // m in (sqrt(1/2), sqrt(2)]: the exponent is one more above sqrt(2)
+    const uint32_t bits = __float_as_uint(w);
+    const uint32_t e = (bits + (0x00800000u - 0x003504f4u)) >> 23;
+    const float f = __uint_as_float(bits - (e << 23) + 0x3f800000u) - 1.0f;
+    const float d = 2.0f + f;
+    const float inv = tgm_rcp(d);
+    const float q = f * inv;
+    const float s = fmaf(fmaf(-q, d, f), inv, q);
+    const float z = s * s;
+    float t = 0x1.c71c72p-4f;
+    t = fmaf(t, z, 0x1.24924ap-3f);
+    t = fmaf(t, z, 0x1.99999ap-3f);
+    t = fmaf(t, z, 0x1.555556p-2f);
+    const float two_s = s + s;
+    const float logm = fmaf(two_s * z, t, two_s);
+    const float ef = (float)((int)e - 127);
+    const float lg = fmaf(ef, TGM_LN2_HI, fmaf(ef, TGM_LN2_LO, logm));
+    const float h = lg * kSoftmaxInvScale;
+    return kx < 30.0f ? fmaf(fmaf(-h, kSoftmaxScale, lg), kSoftmaxInvScale, h) : x;
+}
+
+// softmax of both halves.
+__device__ __forceinline__ F2 softmax2(F2 x)
+{
+    const F2 kx = mul2(x, f2(kSoftmaxScale));
+    const F2 y = f2(fminf(fmaxf(lo(kx), -87.0f), 30.0f), fminf(fmaxf(hi(kx), -87.0f), 30.0f));
+    const F2 shifted = add2(mul2(y, f2(TGM_LOG2E)), f2(0x1.8p+23f));
+    const F2 nk = mul2(add2(shifted, f2(-0x1.8p+23f)), f2(-1.0f));
+    const F2 r = fma2(nk, f2(TGM_LN2_LO), fma2(nk, f2(TGM_LN2_HI), y));
+    F2 p = f2(0x1.a01a02p-13f);
+    p = fma2(p, r, f2(0x1.6c16c2p-10f));
+    p = fma2(p, r, f2(0x1.111112p-7f));
+    p = fma2(p, r, f2(0x1.555556p-5f));
+    p = fma2(p, r, f2(0x1.555556p-3f));
+    p = fma2(p, r, f2(0.5f));
+    p = fma2(p, r, f2(1.0f));
+    p = fma2(p, r, f2(1.0f));
+    const F2 scale = f2(__uint_as_float((__float_as_uint(lo(shifted)) << 23) + 0x3f800000u),
+                        __uint_as_float((__float_as_uint(hi(shifted)) << 23) + 0x3f800000u));
+    const F2 w = add2(f2(1.0f), mul2(p, scale));
+    const uint32_t wa = __float_as_uint(lo(w)), wb = __float_as_uint(hi(w));
+    const uint32_t ea = (wa + (0x00800000u - 0x003504f4u)) >> 23, eb = (wb + (0x00800000u - 0x003504f4u)) >> 23;
+    const F2 f = add2(f2(__uint_as_float(wa - (ea << 23) + 0x3f800000u), __uint_as_float(wb - (eb << 23) + 0x3f800000u)),
+                      f2(-1.0f));
+    const F2 d = add2(f2(2.0f), f);
+    const F2 inv = f2(tgm_rcp(lo(d)), tgm_rcp(hi(d)));
+    const F2 q = mul2(f, inv);
+    const F2 s = fma2(fma2(f2(-lo(q), -hi(q)), d, f), inv, q);
+    const F2 z = mul2(s, s);
+    F2 t = f2(0x1.c71c72p-4f);
+    t = fma2(t, z, f2(0x1.24924ap-3f));
+    t = fma2(t, z, f2(0x1.99999ap-3f));
+    t = fma2(t, z, f2(0x1.555556p-2f));
+    const F2 two_s = add2(s, s);
+    const F2 logm = fma2(mul2(two_s, z), t, two_s);
+    const F2 ef = f2((float)((int)ea - 127), (float)((int)eb - 127));
+    const F2 lg = fma2(ef, f2(TGM_LN2_HI), fma2(ef, f2(TGM_LN2_LO), logm));
+    const F2 h = mul2(lg, f2(kSoftmaxInvScale));
+    const F2 v = fma2(fma2(f2(-lo(h), -hi(h)), f2(kSoftmaxScale), lg), f2(kSoftmaxInvScale), h);
+    return f2(lo(kx) < 30.0f ? lo(v) : lo(x), hi(kx) < 30.0f ? hi(v) : hi(x));
 }
 
 // local.py:91-120 from folded coefficients (sh_fold): the field the
