@@ -376,16 +376,35 @@ cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels
     return cudaGetLastError();
 }
 
+// Row `thread` of the block's rows of n_params floats (zero beyond them), read
+// through dynamic shared memory of blockDim.x rows: the rows are one piece of
+// global memory, but a thread's own row is 180 bytes from its neighbour's.
+template <int CP>
+__device__ __forceinline__ void block_rows(const float* __restrict__ params, uint32_t n_params, uint32_t n,
+                                           float (&raw)[CP])
+{
+    extern __shared__ float block_rows_shared[];
+    const size_t first = (size_t)blockIdx.x * blockDim.x;
+    const uint32_t rows = n - first < blockDim.x ? (uint32_t)(n - first) : blockDim.x;
+    for (uint32_t q = threadIdx.x; q < rows * n_params; q += blockDim.x)     // all copies in flight at once
+        __pipeline_memcpy_async(block_rows_shared + q, params + first * n_params + q, sizeof(float));
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < CP; ++k)
+        raw[k] = (uint32_t)k < n_params && threadIdx.x < rows ? block_rows_shared[threadIdx.x * n_params + k] : 0.0f;
+}
+
 template <int MODEL, int LMAX>
 __global__ void local_evaluate_kernel(const float* __restrict__ params, uint32_t n_params,
                                       const float4* __restrict__ o, uint32_t n, float* __restrict__ out)
 {
     constexpr int CP = MODEL == kModelDTI ? 6 : n_coef_full(LMAX);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     float raw[CP], c[CP];
-#pragma unroll
-    for (int k = 0; k < CP; ++k) raw[k] = (uint32_t)k < n_params ? params[(size_t)i * n_params + k] : 0.0f;
+    block_rows<CP>(params, n_params, n, raw);
+    if (i >= n) return;
     model_coefficients<MODEL, LMAX, CP>(raw, c);
     const float4 v = o[i];
     const Frame f = frame_of(v.x, v.y, v.z);
@@ -402,10 +421,9 @@ __global__ void update_orientation_kernel(AlgoParams a, uint32_t rng_seed, uint6
 {
     constexpr int CP = MODEL == kModelDTI ? 6 : n_coef_full(LMAX);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     float raw[CP], c[CP];
-#pragma unroll
-    for (int k = 0; k < CP; ++k) raw[k] = (uint32_t)k < n_params ? params[(size_t)i * n_params + k] : 0.0f;
+    block_rows<CP>(params, n_params, n, raw);
+    if (i >= n) return;
     model_coefficients<MODEL, LMAX, CP>(raw, c);
     RngState rng = rng_state(a, rng_init(rng_seed, i), seed_offset + i);
     float4 v = o[i];
@@ -461,16 +479,17 @@ cudaError_t launch_local_evaluate(int model, uint32_t n_params, const float* par
                                   float* out, cudaStream_t stream)
 {
     if (n == 0) return cudaSuccess;
-    const int block = 128, grid = (int)((n + block - 1) / block);
+    const int block = 128, grid = (int)((n - 1) / block + 1);
+    const size_t shared = (size_t)block * n_params * sizeof(float);     // block_rows: at most 23 KB
     if (model == kModelDTI) {
-        local_evaluate_kernel<kModelDTI, 0><<<grid, block, 0, stream>>>(params, n_params, o, n, out);
+        local_evaluate_kernel<kModelDTI, 0><<<grid, block, shared, stream>>>(params, n_params, o, n, out);
     } else {
         switch (lmax_for(n_params)) {
-        case 0: local_evaluate_kernel<kModelSH, 0><<<grid, block, 0, stream>>>(params, n_params, o, n, out); break;
-        case 2: local_evaluate_kernel<kModelSH, 2><<<grid, block, 0, stream>>>(params, n_params, o, n, out); break;
-        case 4: local_evaluate_kernel<kModelSH, 4><<<grid, block, 0, stream>>>(params, n_params, o, n, out); break;
-        case 6: local_evaluate_kernel<kModelSH, 6><<<grid, block, 0, stream>>>(params, n_params, o, n, out); break;
-        case 8: local_evaluate_kernel<kModelSH, 8><<<grid, block, 0, stream>>>(params, n_params, o, n, out); break;
+        case 0: local_evaluate_kernel<kModelSH, 0><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
+        case 2: local_evaluate_kernel<kModelSH, 2><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
+        case 4: local_evaluate_kernel<kModelSH, 4><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
+        case 6: local_evaluate_kernel<kModelSH, 6><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
+        case 8: local_evaluate_kernel<kModelSH, 8><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
         default: return cudaErrorInvalidValue;
         }
     }
@@ -482,11 +501,12 @@ static void launch_uo(int algorithm, int grid, int block, cudaStream_t stream, c
                       uint64_t seed_offset, const float* params, uint32_t n_params, const float4* o, uint32_t n,
                       float4* out)
 {
+    const size_t shared = (size_t)block * n_params * sizeof(float);     // block_rows: at most 23 KB
     if (algorithm == kTransport)
-        update_orientation_kernel<M, L, kTransport><<<grid, block, 0, stream>>>(a, rng_seed, seed_offset, params,
+        update_orientation_kernel<M, L, kTransport><<<grid, block, shared, stream>>>(a, rng_seed, seed_offset, params,
                                                                                 n_params, o, n, out);
     else
-        update_orientation_kernel<M, L, kDiffusion><<<grid, block, 0, stream>>>(a, rng_seed, seed_offset, params,
+        update_orientation_kernel<M, L, kDiffusion><<<grid, block, shared, stream>>>(a, rng_seed, seed_offset, params,
                                                                                 n_params, o, n, out);
 }
 
