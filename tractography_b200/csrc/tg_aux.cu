@@ -354,6 +354,33 @@ __global__ void __launch_bounds__(128) fold_field_kernel(const float4* __restric
     }
 }
 
+__global__ void __launch_bounds__(256) pad_field_kernel(const float* __restrict__ packed, float4* __restrict__ padded,
+                                                        uint64_t n_quads, uint32_t n_params, uint32_t quads)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_quads;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = i / quads;
+        const uint32_t k = (uint32_t)(i - v * quads) * 4;
+        const float* row = packed + v * n_params;
+        padded[i] = make_float4(k < n_params ? row[k] : 0.0f, k + 1 < n_params ? row[k + 1] : 0.0f,
+                                k + 2 < n_params ? row[k + 2] : 0.0f, k + 3 < n_params ? row[k + 3] : 0.0f);
+    }
+}
+
+cudaError_t launch_pad_field(const float* packed, float* padded, uint64_t n_voxels, uint32_t n_params, uint32_t cpad,
+                             cudaStream_t stream)
+{
+    if (n_voxels == 0) return cudaSuccess;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint64_t quads = n_voxels * (cpad / 4);
+    const uint64_t want = (quads + 255) / 256, full = (uint64_t)sms * 32;
+    pad_field_kernel<<<(int)(want < full ? want : full), 256, 0, stream>>>(packed, reinterpret_cast<float4*>(padded), quads,
+                                                                          n_params, cpad / 4);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels, int lmax, cudaStream_t stream)
 {
     if (n_voxels == 0) return cudaSuccess;

@@ -353,18 +353,34 @@ int tg_field_create(int32_t model, const float* values, uint32_t nx, uint32_t ny
     f->d.bytes = nvox * f->d.cpad * sizeof(float);
     cudaStream_t s = as_stream(stream);
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&f->d.data), f->d.bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(f->d.data, 0, f->d.bytes, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpy2DAsync(f->d.data, f->d.cpad * sizeof(float), values, n_parameters * sizeof(float),
-                              n_parameters * sizeof(float), nvox, cudaMemcpyHostToDevice, s);
     // the trackers' copy: SH coefficients folded per voxel, tensors as given
-    if (e == cudaSuccess && model == TG_MODEL_SH) {
+    if (e == cudaSuccess && model == TG_MODEL_SH)
         e = cudaMalloc(reinterpret_cast<void**>(&f->d.folded), f->d.bytes);
-        if (e == cudaSuccess) e = launch_fold_field(f->d.data, f->d.folded, nvox, f->d.lmax, s);
+    // The coefficients go up as they are, in one copy, and are padded on the
+    // device: a strided copy of 24- to 180-byte rows from pageable memory ran at
+    // 0.8 GB/s (96x96x60 at lmax 8: 137 ms of field creation, 9.9 ms so).  The
+    // folded copy's memory holds them until it is written; tensors take scratch,
+    // and the strided copy where there is none.
+    const size_t packed_bytes = nvox * n_parameters * sizeof(float);
+    float* scratch = nullptr;
+    float* packed = f->d.cpad == n_parameters ? f->d.data : f->d.folded;
+    if (e == cudaSuccess && packed == nullptr && cudaMalloc(reinterpret_cast<void**>(&scratch), packed_bytes) == cudaSuccess)
+        packed = scratch;
+    if (e == cudaSuccess && packed == nullptr) {
+        cudaGetLastError();
+        e = cudaMemsetAsync(f->d.data, 0, f->d.bytes, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpy2DAsync(f->d.data, f->d.cpad * sizeof(float), values, n_parameters * sizeof(float),
+                                  n_parameters * sizeof(float), nvox, cudaMemcpyHostToDevice, s);
     } else if (e == cudaSuccess) {
-        f->d.folded = f->d.data;
+        e = cudaMemcpyAsync(packed, values, packed_bytes, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess && packed != f->d.data)
+            e = launch_pad_field(packed, f->d.data, nvox, n_parameters, f->d.cpad, s);
     }
+    if (e == cudaSuccess && model == TG_MODEL_SH) e = launch_fold_field(f->d.data, f->d.folded, nvox, f->d.lmax, s);
+    if (e == cudaSuccess && model == TG_MODEL_DTI) f->d.folded = f->d.data;
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (scratch) cudaFree(scratch);
     if (e != cudaSuccess) {
         if (f->d.folded && f->d.folded != f->d.data) cudaFree(f->d.folded);
         if (f->d.data) cudaFree(f->d.data);

@@ -331,6 +331,9 @@ cudaError_t launch_gather(const float* pool, const int32_t* chunk_next, const in
 // Unit hooks (tg_aux.cu).
 cudaError_t launch_contains(const DomainDev& d, const float4* points, uint32_t n, uint8_t* out,
                             cudaStream_t stream);
+// Rows of n_params floats to rows of cpad, zero beyond (cpad a multiple of 4).
+cudaError_t launch_pad_field(const float* packed, float* padded, uint64_t n_voxels, uint32_t n_params, uint32_t cpad,
+                             cudaStream_t stream);
 // SH fields: the folded copy the trackers read (sh_fold per voxel).
 cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels, int lmax, cudaStream_t stream);
 cudaError_t launch_field_evaluate(const FieldDev& f, const float4* points, uint32_t n, float* out,
