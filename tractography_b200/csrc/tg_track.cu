@@ -251,27 +251,23 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             pp.first_chunk[item] = chunk;
             fill = 0;
             emit_point(pp, chunk, fill, a.x, a.y, a.z);
+            if (s.n >= p.n_steps) {      // a streamline of one point: its seed
+                pp.lengths[item] = s.n;
+                continue;
+            }
             return true;
         }
     };
 
-    const bool takes = (threadIdx.x & 31u) < pp.lanes;
-    live = takes && fetch();
-    while (true) {
-        const unsigned active = __ballot_sync(0xffffffffu, live);
-        if (active == 0u) break;
-        if (pp.carry_out != nullptr && warp_should_compact(active, pp.compact_lanes)) {
-            if (live)
-                lane_save<ALGO != kTransport>(pp.carry_out + atomicAdd(pp.carry_out_count, 1u), s, item, chunk,
-                                              fill);
-            break;
-        }
+    live = (threadIdx.x & 31u) < pp.lanes && fetch();
+    unsigned active = __ballot_sync(0xffffffffu, live);
+    while (active != 0u) {
         // Closed surface: the segment tests of this iteration, done here while
         // the warp is together, so that leaf-list tests are shared out over
         // all its lanes (warp_leaves_hit); same answers as a test per lane.
         int surface = -1;
         if constexpr (DOM == kDomainMesh) {
-            const bool testing = live && s.n < p.n_steps && s.steps < p.max_steps && s.steps > 0u;
+            const bool testing = live && s.steps < p.max_steps && s.steps > 0u;
             uint32_t list = 0;
             int route = 0;
             Segment g;
@@ -285,17 +281,22 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             if (__any_sync(0xffffffffu, route == 1)) hit = warp_leaves_hit(p.mesh, route == 1, g, list);
             if (testing) surface = route == 0 ? 0 : (route == 1 ? (hit ? 1 : 0) : -1);
         }
-        bool refill = false;
-        bool slice_end = false;
         float qx, qy, qz;
-        const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
+        const bool go = live && s.steps < p.max_steps;
         const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz, surface);
-        if (live) {
+        // Most iterations of a fine step end here for the whole warp: nothing
+        // was saved and nobody stopped.
+        const bool event = live && r != 1;
+        if (!__any_sync(0xffffffffu, event)) continue;
+        bool refill = false;
+        if (event) {
             bool done = r == 0;
             bool overflow = false;
+            bool slice_end = false;
             if (r == 2) {
                 if (emit_point(pp, chunk, fill, qx, qy, qz)) {
                     s.n++;
+                    done = s.n >= p.n_steps;
                     // a slice ends on a saved point: no test on the other steps
                     if (SLICE && (s.n & pp.slice_mask) == 0u) slice_end = true;
                 } else {
@@ -317,6 +318,13 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         // waits on a lane of its own warp.
         if (SLICE) __syncwarp();
         if (refill) live = fetch();
+        active = __ballot_sync(0xffffffffu, live);
+        if (pp.carry_out != nullptr && warp_should_compact(active, pp.compact_lanes)) {
+            if (live)
+                lane_save<ALGO != kTransport>(pp.carry_out + atomicAdd(pp.carry_out_count, 1u), s, item, chunk,
+                                              fill);
+            break;
+        }
     }
 }
 
