@@ -85,7 +85,7 @@ struct tg_tracker {
     size_t cap_ring = 0;
     uint32_t* ring_flags = nullptr;    // seq then released, cap_ring each
     size_t cap_ring_flags = 0;
-    unsigned int* ring_ctl = nullptr;  // head, tail, fault, spare
+    unsigned int* ring_ctl = nullptr;  // head, tail, warps that left, streamlines ended, fault
     size_t cap_ring_ctl = 0;
     LaneCarry* carry[kJobKinds + 1][2] = {};
     size_t carry_cap[kJobKinds + 1] = {};
@@ -844,8 +844,8 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
         if (cap > 0xFFFFFFFFull) return fail(TG_ERR_INVALID_ARGUMENT, "too many seeds for time slicing");
         TG_TRY(ensure(&t->ring_items, &t->cap_ring, cap));
         TG_TRY(ensure(&t->ring_flags, &t->cap_ring_flags, 2 * cap));
-        TG_TRY(ensure(&t->ring_ctl, &t->cap_ring_ctl, 4));
-        TG_TRY(cudaMemsetAsync(t->ring_ctl, 0, 4 * sizeof(unsigned int), s));
+        TG_TRY(ensure(&t->ring_ctl, &t->cap_ring_ctl, 8));
+        TG_TRY(cudaMemsetAsync(t->ring_ctl, 0, 8 * sizeof(unsigned int), s));
         pp.ring.items = t->ring_items;
         pp.ring.seq = t->ring_flags;
         pp.ring.released = t->ring_flags + cap;
@@ -859,6 +859,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
         uint32_t slice_points = 1;
         while ((uint64_t)slice_points * 2 <= points && slice_points < (1u << 30)) slice_points *= 2;
         pp.slice_mask = slice_points - 1u;
+        pp.merge_blocks = (uint32_t)sms;
     }
     unsigned int* ccount = t->carry_count + 2 * kJobKinds;
 
@@ -900,7 +901,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
             if (pp.ring.items != nullptr) {
                 // an empty ring for each launch; the fault word spans the run
                 TG_TRY(cudaMemsetAsync(pp.ring.seq, 0, 2 * (size_t)pp.ring.capacity * sizeof(uint32_t), s));
-                TG_TRY(cudaMemsetAsync(pp.ring.ctl, 0, 2 * sizeof(unsigned int), s));
+                TG_TRY(cudaMemsetAsync(pp.ring.ctl, 0, 4 * sizeof(unsigned int), s));
             }
             TG_TRY(launch_track_persistent(field->d, pp, wave_grid, block, s));
             t->launches += 1;
@@ -986,7 +987,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
     unsigned int ring_fault = 0;
     TG_TRY(cudaMemcpyAsync(&steps, t->counters + 1, sizeof steps, cudaMemcpyDeviceToHost, s));
     if (pp.ring.items != nullptr)
-        TG_TRY(cudaMemcpyAsync(&ring_fault, pp.ring.ctl + 2, sizeof ring_fault, cudaMemcpyDeviceToHost, s));
+        TG_TRY(cudaMemcpyAsync(&ring_fault, pp.ring.ctl + 4, sizeof ring_fault, cudaMemcpyDeviceToHost, s));
     TG_TRY(cudaStreamSynchronize(s));
     if (ring_fault != 0u)
         return fail(TG_ERR_CUDA, std::string("time slicing: a bounded wait on the queue of saved streamlines ran "

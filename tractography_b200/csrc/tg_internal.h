@@ -25,9 +25,10 @@ constexpr uint32_t kDefaultSliceSteps = 65536;
 // (taken from ctl[1]) is written to slot t % capacity, published by
 // seq[slot] = t + 1; a lane claims the oldest ticket (ctl[0]) only while it
 // is below ctl[1], and marks the slot free again by released[slot] = t + 1.
-// ctl[2]: nonzero when a bounded wait ran out (1: a slot's wait, 2: a
-// claim's retries; the run then fails).  seq,
-// released and ctl are zero at the launch.  capacity exceeds the number of
+// ctl[2] counts the warps that have left the launch, ctl[3] the streamlines that
+// have ended.  ctl[4]: nonzero when a bounded wait ran out (1: a slot's wait, 2: a
+// claim's retries; the run then fails).  seq, released and ctl[0..3] are zero at
+// the launch.  capacity exceeds the number of
 // streamlines that can be live at once, so a ticket's slot was claimed long
 // before the ticket capacity later reuses it.
 struct TrackRing {
@@ -179,6 +180,7 @@ struct PersistentParams {
     // a long streamline started last setting the end of the launch.
     TrackRing ring;
     uint32_t slice_mask;
+    uint32_t merge_blocks;        // blocks given up at a time at the launch's end: one per SM
 };
 
 // Many jobs queued at once (tg_multi.cu).  Job j covers global seed indices

@@ -129,7 +129,7 @@ __device__ __forceinline__ bool ring_wait(const TrackRing& R, const uint32_t* p,
         if (ld_acquire(p) == want) return true;
         __nanosleep(64);
     }
-    atomicOr(R.ctl + 2, 1u);
+    atomicOr(R.ctl + 4, 1u);
     return false;
 }
 
@@ -189,7 +189,7 @@ __device__ __forceinline__ bool ring_take(const TrackRing& R, Lane& s, uint32_t&
         }
     }
     if (!claimed) {
-        atomicOr(R.ctl + 2, 2u);
+        atomicOr(R.ctl + 4, 2u);
         return false;
     }
     const uint32_t slot = h % R.capacity;
@@ -202,6 +202,50 @@ __device__ __forceinline__ bool ring_take(const TrackRing& R, Lane& s, uint32_t&
     st_release(R.released + slot, h + 1u);
     lane_restore<RNG>(s, c, item, chunk, fill);
     return true;
+}
+
+// The end of a sliced launch.  Once the seeds are gone, streamlines end and leave
+// idle lanes, and a warp costs its scheduler the same with one live lane as with
+// 32.  So the launch gives up its blocks from the last one down, one per SM at a time
+// (blocks are dealt to the SMs in turn): when the live streamlines fit kMergeFill
+// / 32 of the lanes of fewer blocks, the warps of the blocks beyond save theirs to
+// the ring and leave, and idle lanes of the others take them.  A warp looks
+// every kMergeEvents events (a saved point or an end in the warp): lanes that came
+// together by merging no longer save in the same iteration, so seldom is better.
+// 100k SDE seeds in 145x174x145 (about the launch's lanes; mean length half the
+// longest), tracking kernel: 536 ms without merging, 481 / 447 / 440 / 459 / 506 ms
+// with 16 / 128 / 256 / 512 / 1024 events, 473 ms with 256 and 28 of 32 lanes; 250k
+// seeds 623 -> 600 ms; letting any sparse warp leave, whichever its block, 600 ms (the
+// schedulers that kept all their warps set the end).
+//
+// No saved streamline is left behind: a warp that leaves counts itself out
+// (ctl[2]) and looks at the ring afterwards, coming back if something waits; a
+// warp that saved its lanes counts itself out after saving them and comes back if
+// no more than one warp per SM is still in.  Whoever is still in at that moment
+// looks at the ring later.
+constexpr uint32_t kMergeEvents = 256;
+constexpr uint32_t kMergeFill = 30;
+
+// Streamlines waiting in the ring.
+__device__ __forceinline__ bool ring_waiting(const TrackRing& R)
+{
+    return ld_relaxed(R.ctl) < ld_relaxed(R.ctl + 1);
+}
+
+// The warp counts itself out and, when `stay` warps or fewer would remain or (with
+// stay 0) streamlines wait, in again; true when it is out.  One lane's answer for
+// all.
+__device__ __forceinline__ bool warp_leaves(const TrackRing& R, uint32_t stay)
+{
+    int out = 0;
+    if ((threadIdx.x & 31u) == 0u) {
+        __threadfence();
+        const uint32_t left = gridDim.x * (blockDim.x >> 5) - 1u - atomicAdd(R.ctl + 2, 1u);
+        __threadfence();
+        out = stay > 0u ? left > stay : !ring_waiting(R);
+        if (!out) atomicSub(R.ctl + 2, 1u);
+    }
+    return __shfl_sync(0xffffffffu, out, 0) != 0;
 }
 
 // SLICE: compiled with time slicing (pp.ring set) or without, so that the
@@ -246,6 +290,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             if (!chunk_alloc(pp, chunk)) {
                 pp.first_chunk[item] = -1;
                 pp.lengths[item] = kOverflowBit;
+                if (SLICE) atomicAdd(pp.ring.ctl + 3, 1u);
                 continue;
             }
             pp.first_chunk[item] = chunk;
@@ -253,6 +298,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             emit_point(pp, chunk, fill, a.x, a.y, a.z);
             if (s.n >= p.n_steps) {      // a streamline of one point: its seed
                 pp.lengths[item] = s.n;
+                if (SLICE) atomicAdd(pp.ring.ctl + 3, 1u);
                 continue;
             }
             return true;
@@ -261,7 +307,14 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
 
     live = (threadIdx.x & 31u) < pp.lanes && fetch();
     unsigned active = __ballot_sync(0xffffffffu, live);
-    while (active != 0u) {
+    uint32_t events = 0;
+    while (true) {
+        if (active == 0u) {
+            if (!SLICE || pp.carry_out != nullptr || warp_leaves(pp.ring, 0u)) break;
+            live = ring_take<ALGO != kTransport>(pp.ring, s, item, chunk, fill);
+            active = __ballot_sync(0xffffffffu, live);
+            continue;
+        }
         // Closed surface: the segment tests of this iteration, done here while
         // the warp is together, so that leaf-list tests are shared out over
         // all its lanes (warp_leaves_hit); same answers as a test per lane.
@@ -307,6 +360,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             if (done) {
                 pp.lengths[item] = overflow ? (s.n | kOverflowBit) : s.n;
                 if (!overflow && pp.steps_done != nullptr) atomicAdd(pp.steps_done, (unsigned long long)s.steps);
+                if (SLICE) atomicAdd(pp.ring.ctl + 3, 1u);
                 refill = true;
             } else if (SLICE && slice_end && work_waiting(pp, n_items)) {
                 ring_push<ALGO != kTransport>(pp.ring, s, item, chunk, fill);
@@ -319,6 +373,22 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         if (SLICE) __syncwarp();
         if (refill) live = fetch();
         active = __ballot_sync(0xffffffffu, live);
+        if (SLICE && pp.carry_out == nullptr && (++events % kMergeEvents) == 0u && active != 0xffffffffu) {
+            const bool drained = *reinterpret_cast<volatile const unsigned long long*>(pp.item_counter) >= n_items;
+            const unsigned long long left = n_items - ld_relaxed(pp.ring.ctl + 3);
+            const unsigned long long per_block = (blockDim.x >> 5) * kMergeFill * (unsigned long long)pp.merge_blocks;
+            const bool beyond = blockIdx.x >= (left + per_block - 1u) / per_block * pp.merge_blocks &&
+                                ld_relaxed(pp.ring.ctl + 1) < kRingTicketLimit;
+            if (__all_sync(0xffffffffu, drained && beyond)) {
+                if (live) ring_push<ALGO != kTransport>(pp.ring, s, item, chunk, fill);
+                live = false;
+                __syncwarp();
+                if (warp_leaves(pp.ring, pp.merge_blocks)) break;
+            } else if (__any_sync(0xffffffffu, drained && ring_waiting(pp.ring))) {
+                if (!live) live = ring_take<ALGO != kTransport>(pp.ring, s, item, chunk, fill);
+            }
+            active = __ballot_sync(0xffffffffu, live);
+        }
         if (pp.carry_out != nullptr && warp_should_compact(active, pp.compact_lanes)) {
             if (live)
                 lane_save<ALGO != kTransport>(pp.carry_out + atomicAdd(pp.carry_out_count, 1u), s, item, chunk,
