@@ -88,7 +88,9 @@ struct Segment {
     float sx, sy, sz;
     float dx, dy, dz;
     float ix, iy, iz;
-    bool px, py, pz;         // |d| < 1e-12 on that axis (bvh.cl:29)
+    // bits 0-2: |d| < 1e-12 on that axis (bvh.cl:29); bit 3: an infinite d.
+    // Zero: the box test without branches holds.
+    uint32_t axes;
 };
 
 __device__ __forceinline__ Segment make_segment(float sx, float sy, float sz, float ex, float ey, float ez)
@@ -96,9 +98,9 @@ __device__ __forceinline__ Segment make_segment(float sx, float sy, float sz, fl
     Segment g;
     g.sx = sx; g.sy = sy; g.sz = sz;
     g.dx = ex - sx; g.dy = ey - sy; g.dz = ez - sz;
-    g.px = fabsf(g.dx) < 1e-12f;
-    g.py = fabsf(g.dy) < 1e-12f;
-    g.pz = fabsf(g.dz) < 1e-12f;
+    const float ux = fabsf(g.dx), uy = fabsf(g.dy), uz = fabsf(g.dz);
+    g.axes = (ux < 1e-12f ? 1u : 0u) | (uy < 1e-12f ? 2u : 0u) | (uz < 1e-12f ? 4u : 0u) |
+             (fmaxf(ux, fmaxf(uy, uz)) > 0x1.fffffep127f ? 8u : 0u);
     g.ix = rcp_signed(g.dx);
     g.iy = rcp_signed(g.dy);
     g.iz = rcp_signed(g.dz);
@@ -128,15 +130,17 @@ __device__ __forceinline__ bool slab(bool parallel, float s, float inv, float lo
 // split a warp three ways here: t0 only grows and t1 only shrinks, so one
 // comparison at the end says what the comparison after each axis would, and
 // min / max differ from the compare-and-select forms above in nothing but the
-// sign of a zero, which no comparison sees, and NaN: one among the slabs leaves
-// t0 and t1 as they are in both, and a NaN max_t (a hit's t after overflow) stays.
+// sign of a zero, which no comparison sees, and NaN.  Both bounds NaN (a NaN in the
+// segment) leave t0 and t1 as they are in both, and a NaN max_t (a hit's t after
+// overflow) stays.  One NaN alone takes a zero reciprocal, so segments with an
+// infinite extent go through the slabs above.
 __device__ __forceinline__ bool box_hit(const Segment& g, float4 lo, float4 hi, float max_t)
 {
     float t0 = 0.0f, t1 = max_t;
-    if (g.px || g.py || g.pz) {
-        if (!slab(g.px, g.sx, g.ix, lo.x, hi.x, t0, t1)) return false;
-        if (!slab(g.py, g.sy, g.iy, lo.y, hi.y, t0, t1)) return false;
-        return slab(g.pz, g.sz, g.iz, lo.z, hi.z, t0, t1);
+    if (g.axes != 0u) {
+        if (!slab((g.axes & 1u) != 0u, g.sx, g.ix, lo.x, hi.x, t0, t1)) return false;
+        if (!slab((g.axes & 2u) != 0u, g.sy, g.iy, lo.y, hi.y, t0, t1)) return false;
+        return slab((g.axes & 4u) != 0u, g.sz, g.iz, lo.z, hi.z, t0, t1);
     }
     const float ax = (lo.x - g.sx) * g.ix, bx = (hi.x - g.sx) * g.ix;
     const float ay = (lo.y - g.sy) * g.iy, by = (hi.y - g.sy) * g.iy;
@@ -402,7 +406,6 @@ __device__ __forceinline__ bool warp_leaves_hit(const MeshDev& m, bool need, con
         if (lane >= o) incl += v;
     }
     const uint32_t total = __shfl_sync(kFull, incl, 31);
-    const uint32_t flags = (g.px ? 1u : 0u) | (g.py ? 2u : 0u) | (g.pz ? 4u : 0u);
     unsigned hits = 0u;
     for (uint32_t base = 0; base < total; base += 32u) {
         const uint32_t w = base + lane;
@@ -424,10 +427,7 @@ __device__ __forceinline__ bool warp_leaves_hit(const MeshDev& m, bool need, con
         o.ix = __shfl_sync(kFull, g.ix, owner);
         o.iy = __shfl_sync(kFull, g.iy, owner);
         o.iz = __shfl_sync(kFull, g.iz, owner);
-        const uint32_t of = __shfl_sync(kFull, flags, owner);
-        o.px = (of & 1u) != 0u;
-        o.py = (of & 2u) != 0u;
-        o.pz = (of & 4u) != 0u;
+        o.axes = __shfl_sync(kFull, g.axes, owner);
         const uint32_t olist = __shfl_sync(kFull, list, owner);
         bool h = false;
         if (w < total) {

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
             int route = 0;
             Segment g;
             g.sx = g.sy = g.sz = g.dx = g.dy = g.dz = g.ix = g.iy = g.iz = 0.0f;
-            g.px = g.py = g.pz = false;
+            g.axes = 0u;
             if (testing) {
                 route = mesh_route(p.mesh, s.lx, s.ly, s.lz, s.px, s.py, s.pz, list);
                 if (route == 1) g = make_segment(s.lx, s.ly, s.lz, s.px, s.py, s.pz);
