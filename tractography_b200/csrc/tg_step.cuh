@@ -100,11 +100,14 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
         // For a voxel f and f - 0.5 < a < f + 0.5 (open), rint(a) = f and
         // floor(fl(a + 0.5)) = f: the sum lies in [f, f + 1) after rounding
         // (f is representable and a + 0.5 < f + 1 rounds to at most a
-        // value below f + 1 for |a| < 2^22).  So |a - f| < 0.5 for the cached
-        // voxel certifies both unchanged: the difference is exact in that
-        // interval (f = 0, or a and f within a factor of two), and outside
-        // it rounds to no less than 0.5.
-        if (fabsf(ax - s.fvx) < 0.5f && fabsf(ay - s.fvy) < 0.5f && fabsf(az - s.fvz) < 0.5f) return true;
+        // value below f + 1 for |a| < 2^22), except for a = 0.5 - 2^-25, whose
+        // sum is half an ulp below 1 and rounds to 1.  So |a - f| < 0.5 - 2^-25 for
+        // the cached voxel certifies both unchanged: the difference is exact
+        // in that interval (f = 0, or a and f within a factor of two), outside
+        // it rounds to no less than 0.5, and only f = 0 has a value a that
+        // close to 0.5 from it.
+        constexpr float kHalf = 0x1.fffffep-2f;
+        if (fabsf(ax - s.fvx) < kHalf && fabsf(ay - s.fvy) < kHalf && fabsf(az - s.fvz) < kHalf) return true;
         const float vx = floorf(ax + 0.5f), vy = floorf(ay + 0.5f), vz = floorf(az + 0.5f);
         const float fx = rintf(ax), fy = rintf(ay), fz = rintf(az);
         if (!(vx >= 0.0f && vx < (float)p.dgrid.nx && vy >= 0.0f && vy < (float)p.dgrid.ny && vz >= 0.0f &&
