@@ -338,9 +338,17 @@ __global__ void __launch_bounds__(128, (persistent_min_blocks<MODEL, LMAX, DOM>(
         const bool go = live && s.steps < p.max_steps;
         const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz, surface);
         // Most iterations of a fine step end here for the whole warp: nothing
-        // was saved and nobody stopped.
+        // was saved and nobody stopped.  Not in the unsliced surface form: its
+        // steps are coarse, and the vote's second way round the loop costs the
+        // tensor kernels spills at their 80 registers (500k Transport tensor seeds
+        // at step 0.2 in 499,280 triangles: kernel 8.23 ms with 20 / 28 bytes
+        // spilled, 8.12 ms without vote and spills; 200k SDE seeds at 0.05 9.84 and
+        // 9.65 ms).  Sliced launches are those of fine steps (100k tensor seeds at
+        // step 0.001: 270 ms with the vote, 350 ms without).
         const bool event = live && r != 1;
-        if (!__any_sync(0xffffffffu, event)) continue;
+        if constexpr (DOM != kDomainMesh || SLICE) {
+            if (!__any_sync(0xffffffffu, event)) continue;
+        }
         bool refill = false;
         if (event) {
             bool done = r == 0;
