@@ -187,19 +187,23 @@ __device__ __forceinline__ bool locate(const TrackParams& p, Lane& s, float (&c)
 // is false), 1 after a step without a saved point, 2 after a step that saved
 // point q.
 //
-// Called by all 32 lanes of a warp together; lanes without a step to make
+// JOIN: called by all 32 lanes of a warp together; lanes without a step to make
 // pass go = false.  locate() has many exits (voxel unchanged, voxel loaded,
 // stopped), and left to itself the compiler joins its paths only behind the
 // update, which then ran once per path: with a 0.1-voxel step some lane of
 // nearly every warp enters a new voxel on every step, and 11-13 of 32 lanes
 // were active per instruction (~1000 warp instructions per step).  The
 // __syncwarp joins the lanes before the update.
-template <int MODEL, int LMAX, int ALGO, int CPAD, int DOM = kDomainImage>
+//
+// Without JOIN a lane is on its own, for loops in which nothing else brings the
+// warp together: its lanes then drift apart by whole steps, and those that
+// wait for a new voxel do not hold up the rest.
+template <int MODEL, int LMAX, int ALGO, int CPAD, int DOM = kDomainImage, bool JOIN = true>
 __device__ __forceinline__ int track_step(const TrackParams& p, bool go, Lane& s, float (&c)[CPAD],
                                           float& qx, float& qy, float& qz, int surface = -1)
 {
     if (go) go = locate<MODEL, LMAX, CPAD, DOM>(p, s, c, surface);
-    __syncwarp();
+    if (JOIN) __syncwarp();
     if (!go) return 0;
     update_orientation<MODEL, LMAX, ALGO>(p.algo, c, s.ox, s.oy, s.oz, s.rng, s.steps);
     s.steps += 1u;
