@@ -58,7 +58,20 @@ constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
 uint32_t* g_scratch_addr[kMaxDevices] = {};
 
-template <int MODEL, int LMAX, int ALGO, int DOM>
+// REFILL: more streamlines than lanes.  Without it each lane tracks one, on its
+// own (track_step without JOIN): nothing waits for a lane's new voxel but that
+// lane.  32^3 volume, 2000 seeds, lmax 8: Transport 0.35 ms, 0.43 ms with the warp
+// joined on every step; SDE 1.42 and 1.75 ms.
+//
+// With it a lane that ends takes the next streamline while its warp goes on,
+// and the warp is joined on every step: SDE streamlines differ in length, and
+// lanes on their own took 300,000 of them in 10.7 ms, joined in 6.5 ms.  Transport
+// streamlines mostly run to the full length together, and from lmax 6 on, where
+// a warp waits longest for a voxel, joining costs more than it gives except
+// where the last few do not fill the GPU again (lmax 8, own / joined: 100,000 seeds
+// 1.11 / 0.97 ms, 150,000 1.35 / 1.61, 300,000 2.59 / 2.73, mask on its own grid
+// 2.86 / 3.28; lmax 4: 300,000 1.57 / 1.21).
+template <int MODEL, int LMAX, int ALGO, int DOM, bool REFILL>
 __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams p, const float4* __restrict__ seeds,
                                                                      uint32_t n_seeds, uint32_t batch_size,
                                                                      uint64_t seed_offset, uint32_t lanes,
@@ -87,19 +100,36 @@ __global__ void __launch_bounds__(128) track_persistent_dense_kernel(TrackParams
         line[0] = a;
         return true;
     };
-    bool live = (threadIdx.x & 31u) < lanes && fetch();
-    while (__any_sync(0xffffffffu, live)) {
-        float qx, qy, qz;
-        const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
-        const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz);
-        if (!live) continue;
-        if (r == 2) {
-            line[s.n] = make_float4(qx, qy, qz, 1.0f);
-            s.n++;
+    if constexpr (REFILL && !(ALGO == kTransport && CPAD > 16)) {
+        bool live = (threadIdx.x & 31u) < lanes && fetch();
+        while (__any_sync(0xffffffffu, live)) {
+            float qx, qy, qz;
+            const bool go = live && s.n < p.n_steps && s.steps < p.max_steps;
+            const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM>(p, go, s, c, qx, qy, qz);
+            if (!live) continue;
+            if (r == 2) {
+                line[s.n] = make_float4(qx, qy, qz, 1.0f);
+                s.n++;
+            }
+            if (r == 0) {
+                lengths[item] = s.n;
+                live = fetch();
+            }
         }
-        if (r == 0) {
+    } else {
+        if ((threadIdx.x & 31u) >= lanes) return;
+        while (fetch()) {
+            while (s.n < p.n_steps && s.steps < p.max_steps) {
+                float qx, qy, qz;
+                const int r = track_step<MODEL, LMAX, ALGO, CPAD, DOM, false>(p, true, s, c, qx, qy, qz);
+                if (r == 0) break;
+                if (r == 2) {
+                    line[s.n] = make_float4(qx, qy, qz, 1.0f);
+                    s.n++;
+                }
+            }
             lengths[item] = s.n;
-            live = fetch();
+            if (!REFILL) break;
         }
     }
 }
@@ -109,18 +139,26 @@ cudaError_t launch_variant(const TrackParams& p, const float4* seeds, uint32_t n
                            uint64_t seed_offset, uint32_t* scratch, float4* out, uint32_t* lengths,
                            cudaStream_t stream)
 {
-    int dev = 0, sms = 0, blocks = 0;
+    int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, track_persistent_dense_kernel<M, L, A, D>, 128, 0);
     if (e != cudaSuccess) return e;
     sms = sms > 0 ? sms : 1;
-    blocks = blocks > 0 ? blocks : 1;
-    const uint32_t lanes = spread_lanes(n, sms, blocks);
-    track_persistent_dense_kernel<M, L, A, D><<<spread_blocks(n, lanes, sms, blocks), 128, 0, stream>>>(
-        p, seeds, n, batch_size, seed_offset, lanes, scratch, out, lengths);
-    return cudaGetLastError();
+    auto start = [&](auto kernel, bool refill) {
+        int blocks = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, 128, 0);
+        if (e != cudaSuccess) return true;
+        blocks = blocks > 0 ? blocks : 1;
+        const uint32_t lanes = spread_lanes(n, sms, blocks);
+        const int grid = spread_blocks(n, lanes, sms, blocks);
+        if (!refill && (uint64_t)grid * 4 * lanes < n) return false;
+        kernel<<<grid, 128, 0, stream>>>(p, seeds, n, batch_size, seed_offset, lanes, scratch, out, lengths);
+        e = cudaGetLastError();
+        return true;
+    };
+    if (!start(track_persistent_dense_kernel<M, L, A, D, false>, false))
+        start(track_persistent_dense_kernel<M, L, A, D, true>, true);
+    return e;
 }
 
 cudaError_t launch(int model, int lmax, int algo, const TrackParams& p, const float4* seeds, uint32_t n,
