@@ -13,7 +13,7 @@ from tractography_b200._lib import LIB_PATH
 pytestmark = pytest.mark.gpu
 
 ARGUMENTS = {"tgm_rcp": 250 << 23, "rcp_signed": 1 << 32, "sqrt_pos2_draws": (1 << 24) - 1,
-             "sqrt_pos2_mantissas": 2 << 23, "log_pos2": (1 << 24) - 1, "cos2pi_2": 1 << 32,
+             "sqrt_pos": 1 << 24, "sqrt_pos2_mantissas": 2 << 23, "log_pos2": (1 << 24) - 1, "cos2pi_2": 1 << 32,
              "exps2": 0x3f800001, "softmax": 1 << 32}
 
 

@@ -51,6 +51,14 @@ struct RootOfDraw {          // i = 1 .. 2^24 - 1: Box-Muller's uniform in 2^-24
     }
 };
 
+struct RootOfCounterDraw {   // i = 1 .. 2^24: the counter-based draw's uniform in 2^-24
+    static __device__ bool bad(uint64_t i)
+    {
+        const float x = -2.0f * tgm_log_pos((float)i * 0x1p-24f);
+        return differs(sqrt_pos(x), sqrtf(x));
+    }
+};
+
 struct RootOfMantissa {      // i: the bits of x in [1, 4)
     static __device__ bool bad(uint64_t i)
     {
@@ -137,6 +145,7 @@ int main()
     const bool ok = run<Reciprocal>("tgm_rcp", 0x01000000u, 0x7e000000u, d_bad) &&           // 2^-125 .. 2^125
                     run<ReciprocalSigned>("rcp_signed", 0, all, d_bad) &&
                     run<RootOfDraw>("sqrt_pos2_draws", 1, 1u << 24, d_bad) &&
+                    run<RootOfCounterDraw>("sqrt_pos", 1, (1u << 24) + 1, d_bad) &&
                     run<RootOfMantissa>("sqrt_pos2_mantissas", 0x3f800000u, 0x40800000u, d_bad) &&
                     run<LogOfDraw>("log_pos2", 1, 1u << 24, d_bad) &&
                     run<CosineOfDraw>("cos2pi_2", 0, all, d_bad) &&

@@ -172,6 +172,17 @@ __device__ __forceinline__ F2 sqrt_pos2(F2 x)
     return fma2(r, h, g);
 }
 
+// The same for one value, or a zero (u = 1, which the counter-based draws
+// reach), which is its own root.
+__device__ __forceinline__ float sqrt_pos(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float g = x * y;
+    const float root = fmaf(fmaf(-g, g, x), 0.5f * y, g);
+    return x > 0.0f ? root : x;
+}
+
 // Two draws of randn, evaluated together: one pass of pairwise arithmetic
 // instead of two, and one test for randn's rejection of u <= 0, which happens
 // once in 2^23 pairs (the draws then move up and the next ones follow).
@@ -218,7 +229,10 @@ __device__ __forceinline__ void philox_normal2(uint64_t key, uint64_t index, uin
                                   make_uint2((uint32_t)key, (uint32_t)(key >> 32)));
     const float u1 = (float)((w.x >> 8) + 1u) * 0x1p-24f;
     const float u2 = (float)(w.y >> 8) * 0x1p-24f;
-    const float radius = sqrtf(-2.0f * tgm_log_pos(u1));
+    // sqrtf's bits (sqrt_pos) without its branch, which kept the draw from
+    // overlapping the model's evaluation: 2000 seeds at lmax 8 in the
+    // dense tracker 1.69 -> 1.60 ms.
+    const float radius = sqrt_pos(-2.0f * tgm_log_pos(u1));
     float s, c;
     tgm_sincosf(TGM_TWO_PI * u2, &s, &c);
     *n1 = radius * c;
