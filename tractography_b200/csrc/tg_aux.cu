@@ -403,24 +403,45 @@ cudaError_t launch_fold_field(const float* raw, float* folded, uint64_t n_voxels
     return cudaGetLastError();
 }
 
-// Row `thread` of the block's rows of n_params floats (zero beyond them), read
-// through dynamic shared memory of blockDim.x rows: the rows are one piece of
-// global memory, but a thread's own row is 180 bytes from its neighbour's.
+// A thread's row of n_params floats (zero beyond them).  Rows of more than six
+// floats (kStagedRows) go through dynamic shared memory of blockDim.x rows: they
+// are one piece of global memory, but a thread's own row is 180 bytes from its
+// neighbour's.  A row of up to 24 bytes shares its sectors with its neighbours',
+// and staging it cost more than it gave (4M rows, read directly / staged: tensor
+// values 35.6 / 41.9 us, tensor updates 38.1 / 51.6 us, lmax 2 values 38.9 / 50.2 us).
 template <int CP>
-__device__ __forceinline__ void block_rows(const float* __restrict__ params, uint32_t n_params, uint32_t n,
-                                           float (&raw)[CP])
+constexpr bool kStagedRows = CP > 6;
+
+template <int MODEL, int LMAX>
+size_t row_bytes(int block, uint32_t n_params)      // load_row's shared memory: at most 23 KB
 {
-    extern __shared__ float block_rows_shared[];
-    const size_t first = (size_t)blockIdx.x * blockDim.x;
-    const uint32_t rows = n - first < blockDim.x ? (uint32_t)(n - first) : blockDim.x;
-    for (uint32_t q = threadIdx.x; q < rows * n_params; q += blockDim.x)     // all copies in flight at once
-        __pipeline_memcpy_async(block_rows_shared + q, params + first * n_params + q, sizeof(float));
-    __pipeline_commit();
-    __pipeline_wait_prior(0);
-    __syncthreads();
+    constexpr int CP = MODEL == kModelDTI ? 6 : n_coef_full(LMAX);
+    return kStagedRows<CP> ? (size_t)block * n_params * sizeof(float) : 0;
+}
+
+// Row i, the thread's; false past the end.  Called by the whole block.
+template <int CP>
+__device__ __forceinline__ bool load_row(const float* __restrict__ params, uint32_t n_params, uint32_t n, uint32_t i,
+                                         float (&raw)[CP])
+{
+    if constexpr (kStagedRows<CP>) {
+        extern __shared__ float staged_rows[];
+        const size_t first = (size_t)blockIdx.x * blockDim.x;
+        const uint32_t rows = n - first < blockDim.x ? (uint32_t)(n - first) : blockDim.x;
+        for (uint32_t q = threadIdx.x; q < rows * n_params; q += blockDim.x)     // all copies in flight at once
+            __pipeline_memcpy_async(staged_rows + q, params + first * n_params + q, sizeof(float));
+        __pipeline_commit();
+        __pipeline_wait_prior(0);
+        __syncthreads();
+        if (i >= n) return false;
 #pragma unroll
-    for (int k = 0; k < CP; ++k)
-        raw[k] = (uint32_t)k < n_params && threadIdx.x < rows ? block_rows_shared[threadIdx.x * n_params + k] : 0.0f;
+        for (int k = 0; k < CP; ++k) raw[k] = (uint32_t)k < n_params ? staged_rows[threadIdx.x * n_params + k] : 0.0f;
+    } else {
+        if (i >= n) return false;
+#pragma unroll
+        for (int k = 0; k < CP; ++k) raw[k] = (uint32_t)k < n_params ? params[(size_t)i * n_params + k] : 0.0f;
+    }
+    return true;
 }
 
 template <int MODEL, int LMAX>
@@ -430,8 +451,7 @@ __global__ void local_evaluate_kernel(const float* __restrict__ params, uint32_t
     constexpr int CP = MODEL == kModelDTI ? 6 : n_coef_full(LMAX);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float raw[CP], c[CP];
-    block_rows<CP>(params, n_params, n, raw);
-    if (i >= n) return;
+    if (!load_row<CP>(params, n_params, n, i, raw)) return;
     model_coefficients<MODEL, LMAX, CP>(raw, c);
     const float4 v = o[i];
     const Frame f = frame_of(v.x, v.y, v.z);
@@ -449,8 +469,7 @@ __global__ void update_orientation_kernel(AlgoParams a, uint32_t rng_seed, uint6
     constexpr int CP = MODEL == kModelDTI ? 6 : n_coef_full(LMAX);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float raw[CP], c[CP];
-    block_rows<CP>(params, n_params, n, raw);
-    if (i >= n) return;
+    if (!load_row<CP>(params, n_params, n, i, raw)) return;
     model_coefficients<MODEL, LMAX, CP>(raw, c);
     RngState rng = rng_state(a, rng_init(rng_seed, i), seed_offset + i);
     float4 v = o[i];
@@ -507,18 +526,23 @@ cudaError_t launch_local_evaluate(int model, uint32_t n_params, const float* par
 {
     if (n == 0) return cudaSuccess;
     const int block = 128, grid = (int)((n - 1) / block + 1);
-    const size_t shared = (size_t)block * n_params * sizeof(float);     // block_rows: at most 23 KB
     if (model == kModelDTI) {
-        local_evaluate_kernel<kModelDTI, 0><<<grid, block, shared, stream>>>(params, n_params, o, n, out);
+        local_evaluate_kernel<kModelDTI, 0><<<grid, block, 0, stream>>>(params, n_params, o, n, out);
     } else {
+#define TG_EVALUATE(L)                                                                                              \
+    case L:                                                                                                        \
+        local_evaluate_kernel<kModelSH, L><<<grid, block, row_bytes<kModelSH, L>(block, n_params), stream>>>(       \
+            params, n_params, o, n, out);                                                                          \
+        break;
         switch (lmax_for(n_params)) {
-        case 0: local_evaluate_kernel<kModelSH, 0><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
-        case 2: local_evaluate_kernel<kModelSH, 2><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
-        case 4: local_evaluate_kernel<kModelSH, 4><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
-        case 6: local_evaluate_kernel<kModelSH, 6><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
-        case 8: local_evaluate_kernel<kModelSH, 8><<<grid, block, shared, stream>>>(params, n_params, o, n, out); break;
+            TG_EVALUATE(0)
+            TG_EVALUATE(2)
+            TG_EVALUATE(4)
+            TG_EVALUATE(6)
+            TG_EVALUATE(8)
         default: return cudaErrorInvalidValue;
         }
+#undef TG_EVALUATE
     }
     return cudaGetLastError();
 }
@@ -528,7 +552,7 @@ static void launch_uo(int algorithm, int grid, int block, cudaStream_t stream, c
                       uint64_t seed_offset, const float* params, uint32_t n_params, const float4* o, uint32_t n,
                       float4* out)
 {
-    const size_t shared = (size_t)block * n_params * sizeof(float);     // block_rows: at most 23 KB
+    const size_t shared = row_bytes<M, L>(block, n_params);
     if (algorithm == kTransport)
         update_orientation_kernel<M, L, kTransport><<<grid, block, shared, stream>>>(a, rng_seed, seed_offset, params,
                                                                                 n_params, o, n, out);
