@@ -209,6 +209,12 @@ int tg_tracker_run_jobs(tg_tracker* tracker, const tg_job* jobs, uint32_t n_jobs
  * No reference counterpart: instrumentation for the benchmark. */
 int tg_tracker_stats(const tg_tracker* tracker, float* kernel_ms, uint32_t* waves, uint32_t* launches);
 
+/* Streamlines that a lane saved for another to go on with in the last launch of
+ * the last tg_tracker_run: slices that ended while other work waited, and the
+ * streamlines of blocks given up at the launch's end (0 without time slicing).
+ * No reference counterpart: instrumentation for the tests. */
+int tg_tracker_handovers(const tg_tracker* tracker, uint32_t* handovers);
+
 /* Launch shape and tail compaction of the tracker's persistent launches.
  * blocks_per_sm: resident blocks of 128 lanes per SM (0 = the occupancy
  * maximum; larger values are capped to it).  Tail compaction: once a launch's

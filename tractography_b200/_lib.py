@@ -48,6 +48,7 @@ EXPORTS = (
     "tg_tracker_run",
     "tg_tracker_run_jobs",
     "tg_tracker_stats",
+    "tg_tracker_handovers",
     "tg_tracker_set_tuning",
     "tg_tracker_get_tuning",
     "tg_tracker_set_slicing",
@@ -157,6 +158,7 @@ def load() -> ctypes.CDLL:
         "tg_tracker_run_jobs": ([P, ctypes.POINTER(Job), U32, ctypes.c_int, P, P, ctypes.POINTER(U64),
                                  ctypes.POINTER(U64), P], ctypes.c_int),
         "tg_tracker_stats": ([P, ctypes.POINTER(F), ctypes.POINTER(U32), ctypes.POINTER(U32)], ctypes.c_int),
+        "tg_tracker_handovers": ([P, ctypes.POINTER(U32)], ctypes.c_int),
         "tg_tracker_set_tuning": ([P, U32, U32, U32], ctypes.c_int),
         "tg_tracker_get_tuning": ([P, ctypes.POINTER(U32), ctypes.POINTER(U32), ctypes.POINTER(U32)], ctypes.c_int),
         "tg_tracker_set_slicing": ([P, U32], ctypes.c_int),

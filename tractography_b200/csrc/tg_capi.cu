@@ -94,6 +94,7 @@ struct tg_tracker {
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     float kernel_ms = 0.0f;
     uint32_t waves = 0;
+    uint32_t handovers = 0;
     uint32_t launches = 0;
 };
 
@@ -675,6 +676,13 @@ int tg_tracker_stats(const tg_tracker* t, float* kernel_ms, uint32_t* waves, uin
     return TG_OK;
 }
 
+int tg_tracker_handovers(const tg_tracker* t, uint32_t* handovers)
+{
+    if (t == nullptr) return fail(TG_ERR_INVALID_ARGUMENT, "tracker is null");
+    if (handovers) *handovers = t->handovers;
+    return TG_OK;
+}
+
 // Carry buffers of one slot for a grid of `lanes` threads (each lane hands
 // over at most one streamline per round).
 static int tracker_carry(tg_tracker* t, int slot, size_t lanes)
@@ -759,6 +767,7 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
     t->kernel_ms = 0.0f;
     t->waves = 0;
     t->launches = 0;
+    t->handovers = 0;
     if (total_points) *total_points = 0;
     if (total_steps) *total_steps = 0;
     if (n_seeds == 0) return TG_OK;
@@ -984,11 +993,13 @@ int tg_tracker_run(tg_tracker* t, const tg_algorithm* algorithm, const tg_domain
         first_wave = false;
     }
     unsigned long long steps = 0;
-    unsigned int ring_fault = 0;
+    unsigned int ring[5] = {};
     TG_TRY(cudaMemcpyAsync(&steps, t->counters + 1, sizeof steps, cudaMemcpyDeviceToHost, s));
     if (pp.ring.items != nullptr)
-        TG_TRY(cudaMemcpyAsync(&ring_fault, pp.ring.ctl + 4, sizeof ring_fault, cudaMemcpyDeviceToHost, s));
+        TG_TRY(cudaMemcpyAsync(ring, pp.ring.ctl, sizeof ring, cudaMemcpyDeviceToHost, s));
     TG_TRY(cudaStreamSynchronize(s));
+    t->handovers = ring[1];
+    const unsigned int ring_fault = ring[4];
     if (ring_fault != 0u)
         return fail(TG_ERR_CUDA, std::string("time slicing: a bounded wait on the queue of saved streamlines ran "
                                              "out (") + ((ring_fault & 1u) ? "slot" : "") +
@@ -1007,6 +1018,7 @@ int tg_tracker_run_jobs(tg_tracker* t, const tg_job* jobs, uint32_t n_jobs, int 
     t->kernel_ms = 0.0f;
     t->waves = 0;
     t->launches = 0;
+    t->handovers = 0;
     if (total_points) *total_points = 0;
     if (total_steps) *total_steps = 0;
     if (n_jobs == 0) return TG_OK;
