@@ -99,6 +99,52 @@ __global__ void cost_randn(const float* in, float* out, int n)
     out[i] = acc;
 }
 
+__global__ void cost_randn2(const float* in, float* out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    Mwc s = rng_init(__float_as_uint(in[i]), (uint32_t)i);
+    float acc = 0.0f;
+    for (int r = 0; r < REPS; ++r) {
+        float a, b;
+        randn2(s, &a, &b);
+        acc += a + b;
+    }
+    out[i] = acc;
+}
+
+__global__ void cost_philox2(const float* in, float* out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t key = __float_as_uint(in[i]);
+    float acc = 0.0f;
+    for (int r = 0; r < REPS; ++r) {
+        float a, b;
+        philox_normal2(key, (uint64_t)i, (uint32_t)r, &a, &b);
+        acc += a + b;
+    }
+    out[i] = acc;
+}
+
+__global__ void cost_rcp(const float* in, float* out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float x = in[i];
+    for (int r = 0; r < REPS; ++r) x = tgm_rcp(x * 1.0001f + 0.5f);
+    out[i] = x;
+}
+
+__global__ void cost_sqrt_pos(const float* in, float* out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float x = in[i];
+    for (int r = 0; r < REPS; ++r) x = sqrt_pos(x * 1.0001f + 0.5f);
+    out[i] = x;
+}
+
 __global__ void cost_frame(const float* in, float* out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -200,6 +246,10 @@ int main()
     cost_sqrt<<<grid, block>>>(in, out, n);
     cost_cos2pi<<<grid, block>>>(in, out, n);
     cost_randn<<<grid, block>>>(in, out, n);
+    cost_randn2<<<grid, block>>>(in, out, n);
+    cost_philox2<<<grid, block>>>(in, out, n);
+    cost_rcp<<<grid, block>>>(in, out, n);
+    cost_sqrt_pos<<<grid, block>>>(in, out, n);
     cost_frame<<<grid, block>>>(in, out, n);
     cost_sh8<<<grid, block>>>(in, out, n);
     cost_softplus<<<grid, block>>>(in, out, n);
