@@ -5,7 +5,8 @@
  * that owns the GPU's memory budget and hands plugins fixed buffers at start
  * up, or a latency-bound loop in which cudaMalloc/cudaFree (which may
  * synchronise the device) are not acceptable.  For them this file provides
- * tg_tractogram_noalloc(): the persistent lane-refill tracker writing the
+ * tg_tractogram_noalloc(): a tracker whose lanes take streamlines from a
+ * queue (one each, or more where they outnumber the lanes) and write the
  * reference's dense output into caller buffers, whose only scratch memory
  * (a work-item counter and the per-batch RNG seeds) lives
  * in the file-scope __device__ array below.
